@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -25,78 +26,201 @@ struct FieldArgs {
   ff_mode modes[kMaxModes];
 };
 
-// phi factors and their second derivatives, FishFry.hpp:22-41 and :71-86.
-struct PointFactors {
-  double px, py, pz, dpx, dpy, dpz;
+// phi factors and their second derivatives along one axis, FishFry.hpp:22-41
+// and :71-86: (factor, second derivative) at one coordinate.
+__device__ __forceinline__ double2 factor_x(double x) {
+  const double cx = cos(x), sx = sin(x), ex = exp(sx);
+  return make_double2(cx * ex, -ex * sx * cx * (sx + 3.0));
+}
+__device__ __forceinline__ double2 factor_y(double y) {
+  const double cy = cos(y), sy = sin(y), ey = exp(cy);
+  return make_double2(sy * ey, sy * ey * (sy * sy - 3.0 * cy - 1.0));
+}
+__device__ __forceinline__ double2 factor_z(double z) {
+  const double cz = cos(z), sz = sin(z), ez = exp(cz);
+  return make_double2(cz * ez, ez * (3.0 * sz * sz - cz * cz * cz - 1.0));
+}
+
+// Both field kernels walk tiles of kTileLines (i, j) lines by at most kTileK
+// points along z.  f and phi are sums of products of one-axis factors, and a
+// mode's cosine is cos(A + B) = cos A cos B - sin A sin B with A = kx x + ky y
+// + theta of the line and B = kz z of the point, so a tile evaluates sines,
+// cosines and exponentials once per line and once per k, in shared memory,
+// and a point costs its products and two multiply-adds per mode: the kernels
+// are bound by HBM (no modes) or by the FP64 pipe (64 modes), not by nine
+// FP64 transcendentals per point (and one more per mode).  On one
+// B200, 256^3 FP64 without modes, f and both norms (one write, one read of the
+// field and three calls): 1.67-1.97 ms before, 0.145 ms now, of which about
+// 0.06 ms is launch and wait latency.
+//
+// A block keeps its z chunk (blockIdx.x % columns) and walks the line tiles, so
+// the z tables are formed once per block (once per chunk on lines of more than
+// kSumBlocks chunks).  Thread (w, lane) holds lines
+// 8w .. 8w+7 of the tile at k = lane and lane + 32: its 16 points share 8 line
+// and 2 z table entries per mode, in registers.
+constexpr int kTileLines = 64;
+constexpr int kTileK = 64;
+constexpr int kTileWarpLines = kTileLines / (kSumThreads / 32);
+
+struct FieldTiles {
+  long tiles;     // line tiles
+  int chunks;     // z chunks of kc points
+  int kc;
+  int columns;    // blocks side by side along the chunks (at most kSumBlocks)
+  int walkers;    // blocks per column, sharing its line tiles
 };
 
-__device__ __forceinline__ PointFactors factors(const FieldArgs &a, int i, int j, int k) {
-  PointFactors q;
-  const double x = a.xlo + i * a.dx;
-  const double cx = cos(x), sx = sin(x), ex = exp(sx);
-  q.px = cx * ex;
-  q.dpx = -ex * sx * cx * (sx + 3.0);
-  const double y = a.ylo + j * a.dy;
-  const double cy = cos(y), sy = sin(y), ey = exp(cy);
-  q.py = sy * ey;
-  q.dpy = sy * ey * (sy * sy - 3.0 * cy - 1.0);
-  const double z = a.zlo + k * a.dz;
-  const double cz = cos(z), sz = sin(z), ez = exp(cz);
-  q.pz = cz * ez;
-  q.dpz = ez * (3.0 * sz * sz - cz * cz * cz - 1.0);
-  return q;
-}
-
-// sum over modes of w_m * cos(k_m . x + theta_m), w_m = a_m (f) or -a_m/|k_m|^2 (phi)
-__device__ __forceinline__ double modes_sum(const FieldArgs &a, int i, int j, int k, bool solution) {
-  double v = 0.0;
-  const double x = a.xlo + i * a.dx, y = a.ylo + j * a.dy, z = a.zlo + k * a.dz;
+// Values of the tile's 16 points of this thread: f (solution = false) or phi,
+// summed as the point-by-point formulas are (FishFry.hpp:44, :87).
+template <bool MODES>
+__device__ __forceinline__ void tile_values(const FieldArgs &a, const double2 *sm, int warp, int lane, bool solution,
+                                            double v[kTileWarpLines][2]) {
+  const double2 *zf = sm, *lx = sm + kTileK, *ly = lx + kTileLines;
+  const double2 *zm = ly + kTileLines, *lm = zm + a.nmodes * kTileK;
+  const double2 z[2] = {zf[lane], zf[lane + 32]};
+#pragma unroll
+  for (int l = 0; l < kTileWarpLines; l++) {
+    const double2 x = lx[warp * kTileWarpLines + l], y = ly[warp * kTileWarpLines + l];
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+      v[l][q] = solution ? x.x * y.x * z[q].x : x.x * y.x * z[q].y + x.x * y.y * z[q].x + x.y * y.x * z[q].x;
+  }
+  if constexpr (!MODES) return;
+  double s[kTileWarpLines][2] = {};
   for (int m = 0; m < a.nmodes; m++) {
-    const ff_mode &md = a.modes[m];
-    const int k2 = md.kx * md.kx + md.ky * md.ky + md.kz * md.kz;
-    if (k2 == 0) continue;
-    const double w = solution ? -md.a / (double)k2 : md.a;
-    v += w * cos((double)md.kx * x + (double)md.ky * y + (double)md.kz * z + md.theta);
+    const double2 b0 = zm[m * kTileK + lane], b1 = zm[m * kTileK + lane + 32];
+#pragma unroll
+    for (int l = 0; l < kTileWarpLines; l++) {
+      const double2 w = lm[m * kTileLines + warp * kTileWarpLines + l];   // weight times (cos A, sin A)
+      s[l][0] = fma(w.x, b0.x, s[l][0]);
+      s[l][1] = fma(w.x, b1.x, s[l][1]);
+      s[l][0] = fma(-w.y, b0.y, s[l][0]);
+      s[l][1] = fma(-w.y, b1.y, s[l][1]);
+    }
   }
-  return v;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_init(const FieldArgs a, T *__restrict__ f) {
-  const long N = (long)a.ni * a.nj * a.nk;
-  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < N; q += (long)gridDim.x * blockDim.x) {
-    const int k = (int)(q % a.nk);
-    const long ij = q / a.nk;
-    const int j = (int)(ij % a.nj);
-    const int i = (int)(ij / a.nj);
-    const PointFactors p = factors(a, i, j, k);
-    double v = p.px * p.py * p.dpz + p.px * p.dpy * p.pz + p.dpx * p.py * p.pz;   // FishFry.hpp:44
-    if (a.nmodes) v += modes_sum(a, i, j, k, false);
-    f[q] = (T)v;
+#pragma unroll
+  for (int l = 0; l < kTileWarpLines; l++) {
+    v[l][0] += s[l][0];
+    v[l][1] += s[l][1];
   }
 }
 
-// Stage 1: per-block {sum|d|, sum d^2, max|d|} over a fixed strided slice of
-// the points, reduced in a fixed tree.  NaN propagates through the max, as the
-// reference's integer atomicMax on the bit pattern does.
-template <typename T>
-__global__ void __launch_bounds__(kSumThreads) k_diff(const FieldArgs a, const T *__restrict__ phi,
+// z tables of a chunk (once per block) and line tables of a line tile.
+// Entries past the chunk or the grid repeat its last point; they are not used.
+__device__ __forceinline__ void z_tables(const FieldArgs &a, double2 *sm, int k0, int kc) {
+  double2 *zf = sm, *zm = sm + kTileK + 2 * kTileLines;
+  for (int q = threadIdx.x; q < kTileK * (1 + a.nmodes); q += kSumThreads) {
+    const int k = k0 + min(q % kTileK, kc - 1);
+    const double z = a.zlo + k * a.dz;
+    if (q < kTileK) {
+      zf[q] = factor_z(z);
+    } else {
+      const int m = q / kTileK - 1;
+      double2 b;
+      sincos((double)a.modes[m].kz * z, &b.y, &b.x);
+      zm[q - kTileK] = b;
+    }
+  }
+}
+__device__ __forceinline__ void line_tables(const FieldArgs &a, double2 *sm, long line0, long nlines, bool solution) {
+  double2 *lx = sm + kTileK, *ly = lx + kTileLines, *lm = ly + kTileLines + a.nmodes * kTileK;
+  for (int q = threadIdx.x; q < kTileLines * (2 + a.nmodes); q += kSumThreads) {
+    const long line = min(line0 + q % kTileLines, nlines - 1);
+    const int i = (int)(line / a.nj);
+    const int j = (int)(line - (long)i * a.nj);
+    const double x = a.xlo + i * a.dx, y = a.ylo + j * a.dy;
+    if (q < kTileLines) {
+      lx[q] = factor_x(x);
+    } else if (q < 2 * kTileLines) {
+      ly[q - kTileLines] = factor_y(y);
+    } else {
+      // weight a (f) or -a / |k|^2 (phi); the zero mode counts as absent
+      const int m = q / kTileLines - 2;
+      const ff_mode &md = a.modes[m];
+      const int k2 = md.kx * md.kx + md.ky * md.ky + md.kz * md.kz;
+      const double w = k2 == 0 ? 0.0 : solution ? -md.a / (double)k2 : md.a;
+      double s, c;
+      sincos((double)md.kx * x + (double)md.ky * y + md.theta, &s, &c);
+      lm[q - 2 * kTileLines] = make_double2(w * c, w * s);
+    }
+  }
+}
+
+template <typename T, bool MODES>
+__global__ void __launch_bounds__(kSumThreads, MODES ? 2 : 4) k_init(const FieldArgs a, const FieldTiles t, T *__restrict__ f) {
+  extern __shared__ double2 smf[];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const long nlines = (long)a.ni * a.nj;
+  for (int chunk = blockIdx.x % t.columns; chunk < t.chunks; chunk += t.columns) {
+    const int k0 = chunk * t.kc, kc = min(t.kc, a.nk - k0);
+    __syncthreads();
+    z_tables(a, smf, k0, kc);
+    for (long tile = blockIdx.x / t.columns; tile < t.tiles; tile += t.walkers) {
+      const long line0 = tile * kTileLines;
+      __syncthreads();
+      line_tables(a, smf, line0, nlines, false);
+      __syncthreads();
+      double v[kTileWarpLines][2];
+      tile_values<MODES>(a, smf, warp, lane, false, v);
+#pragma unroll
+      for (int l = 0; l < kTileWarpLines; l++) {
+        const long line = line0 + warp * kTileWarpLines + l;
+        if (line >= nlines) break;
+        T *row = f + line * a.nk + k0;
+        if (lane < kc) row[lane] = (T)v[l][0];
+        if (lane + 32 < kc) row[lane + 32] = (T)v[l][1];
+      }
+    }
+  }
+}
+
+// Stage 1 of the error sums: per-block {sum|d|, sum d^2, max|d|} over the
+// block's tiles, each thread's points in a fixed order, reduced in a fixed
+// tree; the grid is a function of the dimensions alone, so the sums are
+// reproducible.  NaN propagates through the max, as the reference's integer
+// atomicMax on the bit pattern does.
+template <typename T, bool MODES>
+__global__ void __launch_bounds__(kSumThreads, MODES ? 2 : 3) k_diff(const FieldArgs a, const FieldTiles t, const T *__restrict__ phi,
                                                       double *__restrict__ partial) {
   __shared__ double s1[kSumThreads], s2[kSumThreads], sm[kSumThreads];
-  const long N = (long)a.ni * a.nj * a.nk;
+  extern __shared__ double2 smf[];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const long nlines = (long)a.ni * a.nj;
   double t1 = 0, t2 = 0, tm = 0;
-  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < N; q += (long)gridDim.x * blockDim.x) {
-    const int k = (int)(q % a.nk);
-    const long ij = q / a.nk;
-    const int j = (int)(ij % a.nj);
-    const int i = (int)(ij / a.nj);
-    const PointFactors p = factors(a, i, j, k);
-    double ex = p.px * p.py * p.pz;
-    if (a.nmodes) ex += modes_sum(a, i, j, k, true);
-    const double d = fabs(ex - (phi ? (double)phi[q] : 0.0));   // FishFry.hpp:89
-    t1 += d;
-    t2 += d * d;
-    tm = (d > tm || d != d) ? d : tm;
+  for (int chunk = blockIdx.x % t.columns; chunk < t.chunks; chunk += t.columns) {
+    const int k0 = chunk * t.kc, kc = min(t.kc, a.nk - k0);
+    __syncthreads();
+    z_tables(a, smf, k0, kc);
+    for (long tile = blockIdx.x / t.columns; tile < t.tiles; tile += t.walkers) {
+      const long line0 = tile * kTileLines;
+      // the tile's phi first: its loads are in flight while the tables are formed
+      T p[kTileWarpLines][2];
+#pragma unroll
+      for (int l = 0; l < kTileWarpLines; l++) {
+        const long line = line0 + warp * kTileWarpLines + l;
+        const T *row = phi + line * a.nk + k0;
+        p[l][0] = phi && line < nlines && lane < kc ? row[lane] : (T)0;
+        p[l][1] = phi && line < nlines && lane + 32 < kc ? row[lane + 32] : (T)0;
+      }
+      __syncthreads();
+      line_tables(a, smf, line0, nlines, true);
+      __syncthreads();
+      double v[kTileWarpLines][2];
+      tile_values<MODES>(a, smf, warp, lane, true, v);
+#pragma unroll
+      for (int l = 0; l < kTileWarpLines; l++) {
+        const long line = line0 + warp * kTileWarpLines + l;
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+          if (line < nlines && lane + 32 * q < kc) {
+            const double d = fabs(v[l][q] - (double)p[l][q]);   // FishFry.hpp:89
+            t1 += d;
+            t2 += d * d;
+            tm = (d > tm || d != d) ? d : tm;
+          }
+        }
+      }
+    }
   }
   s1[threadIdx.x] = t1;
   s2[threadIdx.x] = t2;
@@ -171,10 +295,103 @@ static int field_args(const int n[3], const double xlo[3], const double dx[3], i
   return FF_OK;
 }
 
-static unsigned grid_for(long N, int threads) {
-  long b = (N + threads - 1) / threads;
-  return (unsigned)(b < 148L * 32 ? (b < 1 ? 1 : b) : 148L * 32);
+// Launch shape: z chunks of equal length up to kTileK, and as many blocks per
+// chunk as keep the grid within kSumBlocks (8 blocks per SM; one block per SM
+// fits when 64 modes fill its tables).
+static FieldTiles tile_shape(const FieldArgs &a) {
+  FieldTiles t;
+  const long nlines = (long)a.ni * a.nj;
+  t.chunks = (a.nk + kTileK - 1) / kTileK;
+  t.kc = (a.nk + t.chunks - 1) / t.chunks;
+  t.chunks = (a.nk + t.kc - 1) / t.kc;
+  t.columns = t.chunks < kSumBlocks ? t.chunks : kSumBlocks;
+  t.tiles = (nlines + kTileLines - 1) / kTileLines;
+  const int per_column = kSumBlocks / t.columns;
+  t.walkers = per_column < t.tiles ? per_column : (int)t.tiles;
+  return t;
 }
+
+static size_t tile_smem(const FieldArgs &a) {
+  return sizeof(double2) * ((size_t)(1 + a.nmodes) * kTileK + (size_t)(2 + a.nmodes) * kTileLines);
+}
+
+// Lets fn use the tables of kMaxModes modes.
+template <typename F> static int allow_tables(F fn, size_t smem) {
+  if (smem > 48 * 1024 - 3 * kSumThreads * sizeof(double))
+    FF_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(double2) * ((1 + kMaxModes) * kTileK + (2 + kMaxModes) * kTileLines))));
+  return FF_OK;
+}
+
+// Per-block partial sums of |exact phi - phi| into partial[3 * blocks].
+static int launch_diff(const FieldArgs &a, int precision, const void *phi, double *partial, cudaStream_t st,
+                       int *blocks) {
+  const FieldTiles t = tile_shape(a);
+  const size_t smem = tile_smem(a);
+  *blocks = t.columns * t.walkers;
+  auto launch = [&](auto fn, auto *p) -> int {
+    const int rc = allow_tables(fn, smem);
+    if (rc == FF_OK) fn<<<*blocks, kSumThreads, smem, st>>>(a, t, p, partial);
+    return rc;
+  };
+  const bool m = a.nmodes > 0;
+  const double *pd = static_cast<const double *>(phi);
+  const float *pf = static_cast<const float *>(phi);
+  const int rc = precision == FF_FP64 ? (m ? launch(k_diff<double, true>, pd) : launch(k_diff<double, false>, pd))
+                                      : (m ? launch(k_diff<float, true>, pf) : launch(k_diff<float, false>, pf));
+  if (rc != FF_OK) return rc;
+  FF_CUDA(cudaGetLastError());
+  return FF_OK;
+}
+
+// Scratch of ff_error_sums: the partial triples and the final triple of one
+// call.  kSumSlots of them per GPU are part of the module; a call claims one for
+// its duration (it waits for its stream before it returns, so the slot is idle
+// again) and only allocates when all are in use by other threads.  An allocation
+// per call cost more than the kernel: freed memory goes back to the system at the
+// wait, and the next call maps it again (0.4 ms of a 0.8 ms call at 256^3).
+constexpr int kSumSlots = 16;
+constexpr int kSumSlotDoubles = 3 * kSumBlocks + 3;
+static __device__ __align__(256) double g_sum_slots[kSumSlots][kSumSlotDoubles];
+
+class SumScratch {
+ public:
+  explicit SumScratch(cudaStream_t st) : st_(st) {}
+  ~SumScratch() {
+    if (own_) cudaFreeAsync(p_, st_);
+    if (slot_ >= 0) busy(dev_).fetch_and(~(1u << slot_));
+  }
+  SumScratch(const SumScratch &) = delete;
+  SumScratch &operator=(const SumScratch &) = delete;
+  int take(double **out) {
+    FF_CUDA(cudaGetDevice(&dev_));
+    if (dev_ >= 0 && dev_ < kDevices) {
+      for (int q = 0; q < kSumSlots && slot_ < 0; q++)
+        if (!(busy(dev_).fetch_or(1u << q) & (1u << q))) slot_ = q;
+    }
+    if (slot_ >= 0) {
+      void *base = nullptr;
+      FF_CUDA(cudaGetSymbolAddress(&base, g_sum_slots));
+      *out = static_cast<double *>(base) + (size_t)slot_ * kSumSlotDoubles;
+      return FF_OK;
+    }
+    FF_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&p_), kSumSlotDoubles * sizeof(double), st_));
+    own_ = true;
+    *out = p_;
+    return FF_OK;
+  }
+
+ private:
+  static constexpr int kDevices = 64;
+  static std::atomic<unsigned> &busy(int dev) {
+    static std::atomic<unsigned> mask[kDevices] = {};
+    return mask[dev];
+  }
+  cudaStream_t st_;
+  int dev_ = -1, slot_ = -1;
+  bool own_ = false;
+  double *p_ = nullptr;
+};
 
 // ---------------------------------------------------------------------------
 // Error sums without any device allocation.
@@ -187,64 +404,15 @@ static unsigned grid_for(long N, int threads) {
 // file-scope device array instead of a per-call buffer: every GPU that loads
 // this library holds it (about 384 KB) until the process exits.
 //
-// Each block reduces one contiguous chunk of points in a fixed order.  The
-// chunk length is a function of N alone (about N / kNoAllocBlocks, a multiple
-// of kSumThreads), so small grids still spread over every SM and the
-// summation order is the same on every call for a given grid.  The grid is
-// limited to kNoAllocMaxPoints = 2^30 points (1024^3); the array holds the
-// partials of at most kNoAllocMaxChunks blocks plus the final triple.
-constexpr int kNoAllocBlocks = 8 * 148;
+// Each block reduces its tiles in a fixed order; the grid is a function of the
+// dimensions alone, so the summation order is the same on every call for a
+// given grid.  The grid is limited to kNoAllocMaxPoints = 2^30 points (1024^3);
+// the array holds the partials of at most kNoAllocMaxChunks blocks plus the
+// final triple.
 constexpr int kNoAllocMaxChunks = 16384;
 constexpr long kNoAllocMaxPoints = 1L << 30;
+static_assert(kSumBlocks <= kNoAllocMaxChunks, "the fixed array holds every block's partials");
 static __device__ __align__(256) double g_noalloc_partials[3 * kNoAllocMaxChunks + 3];
-
-// Chunk length for a grid of N points: ceil(N / kNoAllocBlocks) rounded up to
-// a multiple of kSumThreads; chunks = ceil(N / chunk) <= kNoAllocBlocks.
-static long noalloc_chunk(long N) {
-  long c = (N + kNoAllocBlocks - 1) / kNoAllocBlocks;
-  return (c + kSumThreads - 1) / kSumThreads * kSumThreads;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kSumThreads) k_diff_chunks(const FieldArgs a, const T *__restrict__ phi,
-                                                             long chunk, double *__restrict__ partial) {
-  __shared__ double s1[kSumThreads], s2[kSumThreads], sm[kSumThreads];
-  const long N = (long)a.ni * a.nj * a.nk;
-  const long q0 = (long)blockIdx.x * chunk;
-  const long q1 = q0 + chunk < N ? q0 + chunk : N;
-  double t1 = 0, t2 = 0, tm = 0;
-  for (long q = q0 + threadIdx.x; q < q1; q += blockDim.x) {
-    const int k = (int)(q % a.nk);
-    const long ij = q / a.nk;
-    const int j = (int)(ij % a.nj);
-    const int i = (int)(ij / a.nj);
-    const PointFactors p = factors(a, i, j, k);
-    double ex = p.px * p.py * p.pz;
-    if (a.nmodes) ex += modes_sum(a, i, j, k, true);
-    const double d = fabs(ex - (phi ? (double)phi[q] : 0.0));
-    t1 += d;
-    t2 += d * d;
-    tm = (d > tm || d != d) ? d : tm;
-  }
-  s1[threadIdx.x] = t1;
-  s2[threadIdx.x] = t2;
-  sm[threadIdx.x] = tm;
-  __syncthreads();
-  for (int w = kSumThreads / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      s1[threadIdx.x] += s1[threadIdx.x + w];
-      s2[threadIdx.x] += s2[threadIdx.x + w];
-      const double o = sm[threadIdx.x + w];
-      if (o > sm[threadIdx.x] || o != o) sm[threadIdx.x] = o;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    partial[3 * blockIdx.x + 0] = s1[0];
-    partial[3 * blockIdx.x + 1] = s2[0];
-    partial[3 * blockIdx.x + 2] = sm[0];
-  }
-}
 
 // Device address of g_noalloc_partials on the current device.  The name is a
 // host-side stand-in, not a device address, so it is looked up once per
@@ -283,10 +451,22 @@ int ff_init_field(const int n[3], const double xlo[3], const double dx[3], int n
   if (rc != FF_OK) return rc;
   if (!f) return set_error(FF_ERR_INVALID, "ff_init_field: null field");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const long N = (long)n[0] * n[1] * n[2];
-  if (precision == FF_FP64) k_init<double><<<grid_for(N, 256), 256, 0, st>>>(a, static_cast<double *>(f));
-  else if (precision == FF_FP32) k_init<float><<<grid_for(N, 256), 256, 0, st>>>(a, static_cast<float *>(f));
-  else return set_error(FF_ERR_INVALID, "ff_init_field: bad precision %d", precision);
+  if (precision != FF_FP64 && precision != FF_FP32)
+    return set_error(FF_ERR_INVALID, "ff_init_field: bad precision %d", precision);
+  const FieldTiles t = tile_shape(a);
+  const size_t smem = tile_smem(a);
+  const unsigned blocks = (unsigned)(t.columns * t.walkers);
+  auto launch = [&](auto fn, auto *p) -> int {
+    const int rc = allow_tables(fn, smem);
+    if (rc == FF_OK) fn<<<blocks, kSumThreads, smem, st>>>(a, t, p);
+    return rc;
+  };
+  const bool m = a.nmodes > 0;
+  double *pd = static_cast<double *>(f);
+  float *pf = static_cast<float *>(f);
+  rc = precision == FF_FP64 ? (m ? launch(k_init<double, true>, pd) : launch(k_init<double, false>, pd))
+                            : (m ? launch(k_init<float, true>, pf) : launch(k_init<float, false>, pf));
+  if (rc != FF_OK) return rc;
   FF_CUDA(cudaGetLastError());
   return FF_OK;
 }
@@ -300,20 +480,20 @@ int ff_error_sums(const int n[3], const double xlo[3], const double dx[3], int n
   if (precision != FF_FP64 && precision != FF_FP32)
     return set_error(FF_ERR_INVALID, "ff_error_sums: bad precision %d", precision);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // scratch: kSumBlocks partial triples and the final triple, stream-ordered
+  SumScratch held(st);
   double *scratch = nullptr;
-  FF_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&scratch), (3 * kSumBlocks + 3) * sizeof(double), st));
-  if (precision == FF_FP64)
-    k_diff<double><<<kSumBlocks, kSumThreads, 0, st>>>(a, static_cast<const double *>(phi), scratch);
-  else
-    k_diff<float><<<kSumBlocks, kSumThreads, 0, st>>>(a, static_cast<const float *>(phi), scratch);
-  k_diff_final<<<1, kSumThreads, 0, st>>>(scratch, kSumBlocks, scratch + 3 * kSumBlocks);
+  rc = held.take(&scratch);
+  if (rc != FF_OK) return rc;
+  int blocks = 0;
+  rc = launch_diff(a, precision, phi, scratch, st, &blocks);
+  if (rc != FF_OK) return rc;
+  k_diff_final<<<1, kSumThreads, 0, st>>>(scratch, blocks, scratch + 3 * kSumBlocks);
   cudaError_t e = cudaGetLastError();
   double host[3] = {0, 0, 0};
   if (e == cudaSuccess) e = cudaMemcpyAsync(host, scratch + 3 * kSumBlocks, sizeof(host), cudaMemcpyDeviceToHost, st);
-  cudaError_t ef = cudaFreeAsync(scratch, st);
-  if (e == cudaSuccess) e = ef;
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  // the scratch is given back (and host read) only when the stream is done with it
+  const cudaError_t es = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = es;
   if (e != cudaSuccess)
     return set_error(FF_ERR_CUDA, "ff_error_sums: %s (%s)", cudaGetErrorName(e), cudaGetErrorString(e));
   sums[0] = host[0];
@@ -335,23 +515,16 @@ int ff_error_sums_noalloc(const int n[3], const double xlo[3], const double dx[3
     return set_error(FF_ERR_UNSUPPORTED,
                      "ff_error_sums_noalloc: %ld points exceed the fixed partial-sum array's limit of %ld points", N,
                      kNoAllocMaxPoints);
-  const long chunk = noalloc_chunk(N);
-  const long chunks = (N + chunk - 1) / chunk;
-  if (chunks > kNoAllocMaxChunks)   // cannot happen for N <= kNoAllocMaxPoints; kept as the array's guard
-    return set_error(FF_ERR_UNSUPPORTED, "ff_error_sums_noalloc: %ld chunks exceed the fixed array", chunks);
   double *partial = nullptr;
   rc = noalloc_partials(&partial);
   if (rc != FF_OK) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // every slot read below is written by this call first: nothing to clear
-  if (precision == FF_FP64)
-    k_diff_chunks<double><<<(unsigned)chunks, kSumThreads, 0, st>>>(a, static_cast<const double *>(phi), chunk,
-                                                                    partial);
-  else
-    k_diff_chunks<float><<<(unsigned)chunks, kSumThreads, 0, st>>>(a, static_cast<const float *>(phi), chunk,
-                                                                   partial);
+  int blocks = 0;
+  rc = launch_diff(a, precision, phi, partial, st, &blocks);
+  if (rc != FF_OK) return rc;
   double *total = partial + 3 * kNoAllocMaxChunks;
-  k_diff_final<<<1, kSumThreads, 0, st>>>(partial, (int)chunks, total);
+  k_diff_final<<<1, kSumThreads, 0, st>>>(partial, blocks, total);
   cudaError_t e = cudaGetLastError();
   double host[3] = {0, 0, 0};
   if (e == cudaSuccess) e = cudaMemcpyAsync(host, total, sizeof(host), cudaMemcpyDeviceToHost, st);
