@@ -6,6 +6,7 @@ Everything is compiled in-tree with nvcc for `-gencode arch=compute_100a,code=sm
 no JIT cache and no other architecture.  Rebuilds only what is out of date.
 """
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -21,9 +22,20 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + ["-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC,-pthread", "-I" + INCLUDE]
 
 LIB_SOURCES = ["ff_solve.cu", "ff_bluestein.cu", "ff_field.cu", "ff_batch.cu", "ff_batch_f64.cu", "ff_batch_f32.cu",
-               "ff_serve.cu", "ff_slab.cu"]
-HEADERS = ["ff_fft.cuh", "ff_tiles.cuh", "ff_status.hpp", "ff_batch.hpp", "ff_batch_dev.cuh", "ff_bluestein.hpp",
-           "ff_plan.hpp"]
+               "ff_serve.cu", "ff_slab.cu", "ff_gen.cu", "ff_gen_f64.cu", "ff_gen_f32.cu"]
+
+
+def _includes(path, seen=None):
+    """The project files that `path` includes by quotes, and what those include."""
+    seen = set() if seen is None else seen
+    with open(path) as f:
+        names = re.findall(r'^\s*#\s*include\s+"([^"]+)"', f.read(), re.M)
+    for name in names:
+        h = os.path.normpath(os.path.join(os.path.dirname(path), name))
+        if os.path.exists(h) and h not in seen:
+            seen.add(h)
+            _includes(h, seen)
+    return seen
 
 
 def _nvcc():
@@ -51,12 +63,12 @@ def _run(cmd, verbose):
 
 def build_lib(verbose=False, force=False):
     srcs = [os.path.join(CSRC, s) for s in LIB_SOURCES]
-    shared = [os.path.join(CSRC, h) for h in HEADERS] + [os.path.join(INCLUDE, "fishfry.h"), os.path.abspath(__file__)]
     objdir = os.path.join(HERE, "lib", "obj")
     os.makedirs(objdir, exist_ok=True)
     objs = [os.path.join(objdir, os.path.basename(s) + ".o") for s in srcs]
-    # a translation unit is rebuilt when it, a shared header or this recipe is newer than its object
-    todo = [(s, o) for s, o in zip(srcs, objs) if force or _stale(o, [s] + shared)]
+    # a translation unit is rebuilt when it, a header it includes or this recipe is newer than its object
+    todo = [(s, o) for s, o in zip(srcs, objs)
+            if force or _stale(o, [s, os.path.abspath(__file__)] + sorted(_includes(s)))]
     if not todo and not _stale(LIB, objs):
         return LIB
     # translation units compile in parallel (each is one nvcc process); each

@@ -7,6 +7,7 @@
 
 #include "ff_bluestein.hpp"
 #include "ff_fft.cuh"
+#include "ff_gen.hpp"
 #include "ff_status.hpp"
 #include "ff_tiles.cuh"
 
@@ -14,7 +15,7 @@ namespace ff {
 
 // Launch shape of a strided pass (one TMA tile per block).
 struct StridedCfg {
-  int N;          // specialised length of the kernel, 0 = runtime plan
+  int N;          // specialised length of the kernel, 0 = generic passes
   int W;          // columns per tile
   int box_rows;   // rows per TMA box (a divisor of n, at most 256)
   size_t smem;    // dynamic shared memory: one tile + alignment slack
@@ -47,8 +48,7 @@ struct ff_plan {
   int *status;
   int *counters;       // fused passes: 2 tickets + 2 x ni plane counts
   int fused;           // 1: three launches (fused z/y passes), 0: five launches
-  int zN;              // z passes: specialised length, 0 = runtime plan
-  bool zbulk;          // z passes: line blocks by bulk copies
+  int zN;              // z passes: specialised length, 0 = generic passes
   int zW, zP;          // z passes: line pairs per block, line pitch in complex values
   size_t zsmem;
   unsigned ztiles;
@@ -64,6 +64,12 @@ struct ff_plan {
   ff::BsAxis<double2> bsd[3];
   ff::BsAxis<float2> bsf[3];
   ff::BsCfg bscfg[5];
+  // axes of 2^a 3^b 5^c 7^d points without a compile-time plan (ff_gen_dev.cuh):
+  // pass arguments and launch shape by axis
+  bool gen[3];
+  ff::GenPass<double2> gpd[3];
+  ff::GenPass<float2> gpf[3];
+  ff::GenShape gshape[3];
   cudaEvent_t ev[FF_MAX_PHASES + 1];
 };
 
@@ -88,6 +94,20 @@ template <typename T> PassArgs<T> pass_args(const ff_plan *p) {
   a.l2_ahead = p->l2_ahead;
   a.wait_iters = p->wait_iters;
   return a;
+}
+
+// The generic passes' arguments of axis d, and their launch (kind as
+// gen_launch numbers it; st: stream).
+template <typename T> GenPass<typename Cplx<T>::type> gen_pass(const ff_plan *p, int d) {
+  if constexpr (sizeof(T) == 8) {
+    GenPass<double2> a = p->gpd[d];
+    a.wait_iters = p->wait_iters;
+    return a;
+  } else {
+    GenPass<float2> a = p->gpf[d];
+    a.wait_iters = p->wait_iters;
+    return a;
+  }
 }
 
 // Tensor map of a half spectrum at `base` (ni planes of nj rows of nh complex

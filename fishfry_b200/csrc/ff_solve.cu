@@ -35,16 +35,14 @@
 namespace ff {
 
 // Lengths with compile-time specialised kernels (fully unrolled stages);
-// every other length runs the same kernels with the plan read at run time.
+// other 2^a 3^b 5^c 7^d lengths take the generic passes (ff_gen_dev.cuh).
 #define FF_FOR_EACH_SPECIAL_N(X) X(64) X(128) X(256) X(512) X(1024)
 
 // ------------------------------------------------- unfused pass kernels
 // (one launch per pass; used when the fused passes are switched off)
-// With BULK (every specialised length, and runtime lengths whose lines are
-// whole 16-byte multiples and whose plan has at least two stages) both z
-// passes move their line blocks both ways with bulk copies; otherwise the
-// threads load the lines, and the inverse stores them.  The spectrum rows
-// always leave (forward) and enter (inverse) as 16-byte multiples.
+// These are the passes of the lengths with compile-time plans; other lengths
+// take the generic passes (ff_gen_dev.cuh).  Both z passes move their line
+// blocks both ways with bulk copies.
 //
 // The z passes run blocks of kZPassThreads = 128 threads on tiles of about
 // 32 KB, six per SM: more, smaller tiles in flight hide each block's inbound
@@ -52,7 +50,7 @@ namespace ff {
 // / 0.385 -> 0.337 / 0.321 ms; FP32 0.223 / 0.223 -> 0.204 / 0.201 ms).
 constexpr int kZPassThreads = 128;
 
-template <typename T, int N, bool BULK>
+template <typename T, int N>
 __global__ void __launch_bounds__(kZPassThreads, 6) k_zfwd(const T *__restrict__ f, typename Cplx<T>::type *spec,
                                                        const PassArgs<T> a, int W, int P) {
   extern __shared__ unsigned char smraw[];
@@ -63,18 +61,18 @@ __global__ void __launch_bounds__(kZPassThreads, 6) k_zfwd(const T *__restrict__
   }
   __syncthreads();
   const long nlines = (long)a.ni * a.nj;
-  if (BULK && threadIdx.x == 0) {
+  if (threadIdx.x == 0) {
     // whole lines are 16-byte multiples here
     const long fl = ((long)blockIdx.x + a.l2_ahead) * (2 * W);
     if (a.l2_ahead > 0 && fl < nlines)
       l2_prefetch(f + fl * a.nk, (uint32_t)(min((long)(2 * W), nlines - fl) * a.nk * sizeof(T)));
   }
   const ZTileIO io{&mbar, 0, a.status, a.wait_iters};
-  z_fwd_tile<T, N, BULK, true, true, kZPassThreads>(f, spec, a, W, P, (long)blockIdx.x * (2 * W), nlines,
+  z_fwd_tile<T, N, true, true, true, kZPassThreads>(f, spec, a, W, P, (long)blockIdx.x * (2 * W), nlines,
                                reinterpret_cast<typename Cplx<T>::type *>(align128(smraw)), io);
 }
 
-template <typename T, int N, bool BULK>
+template <typename T, int N>
 __global__ void __launch_bounds__(kZPassThreads, 6) k_zinv(const typename Cplx<T>::type *spec, T *__restrict__ out,
                                                        const PassArgs<T> a, int W, int P) {
   extern __shared__ unsigned char smraw[];
@@ -87,14 +85,14 @@ __global__ void __launch_bounds__(kZPassThreads, 6) k_zinv(const typename Cplx<T
   const long nlines = (long)a.ni * a.nj;
   // the same L2 hint as the forward pass, on the spectrum rows (contiguous
   // for a block's line pairs)
-  if (BULK && threadIdx.x == 32) {
+  if (threadIdx.x == 32) {
     const long fl = ((long)blockIdx.x + a.l2_ahead) * (2 * W);
     if (a.l2_ahead > 0 && fl < nlines)
       l2_prefetch(spec + fl * a.nhp,
                   (uint32_t)(min((long)(2 * W), nlines - fl) * a.nhp * sizeof(typename Cplx<T>::type)));
   }
   const ZTileIO io{&mbar, 0, a.status, a.wait_iters};
-  z_inv_tile<T, N, BULK, true, kZPassThreads>(spec, out, a, W, P, (long)blockIdx.x * (2 * W), nlines,
+  z_inv_tile<T, N, true, true, kZPassThreads>(spec, out, a, W, P, (long)blockIdx.x * (2 * W), nlines,
                          reinterpret_cast<typename Cplx<T>::type *>(align128(smraw)), io);
 }
 
@@ -396,38 +394,35 @@ static int special_n(int n) {
   return 0;
 }
 
-// bulk: line blocks by bulk copies (always for specialised lengths)
-template <typename T> static ZFwdKernel<T> zfwd_kernel(int N, bool bulk) {
-#define FF_CASE(NN) if (N == NN) return k_zfwd<T, NN, true>;
+template <typename T> static ZFwdKernel<T> zfwd_kernel(int N) {
+#define FF_CASE(NN) if (N == NN) return k_zfwd<T, NN>;
   FF_FOR_EACH_SPECIAL_N(FF_CASE)
 #undef FF_CASE
-  return bulk ? k_zfwd<T, 0, true> : k_zfwd<T, 0, false>;
+  return nullptr;
 }
-template <typename T> static ZInvKernel<T> zinv_kernel(int N, bool bulk) {
-#define FF_CASE(NN) if (N == NN) return k_zinv<T, NN, true>;
+template <typename T> static ZInvKernel<T> zinv_kernel(int N) {
+#define FF_CASE(NN) if (N == NN) return k_zinv<T, NN>;
   FF_FOR_EACH_SPECIAL_N(FF_CASE)
 #undef FF_CASE
-  return bulk ? k_zinv<T, 0, true> : k_zinv<T, 0, false>;
+  return nullptr;
 }
 
 // kind: 0 = y forward, 1 = y inverse, 2 = x (forward, filter, inverse);
-// N: the compile-time plan (0: runtime plan); W: columns per tile row.
+// N: the compile-time plan; W: columns per tile row.
 template <typename T, int N, int W> static StridedKernel<T> strided_nw(int kind) {
   return kind == 0 ? k_strided<T, W, false, false, N>
                    : kind == 1 ? k_strided<T, W, false, true, N> : k_strided<T, W, true, false, N>;
 }
 // Lengths with compile-time strided tiles of 128-byte rows; 1024-point lines
-// take 64-byte rows (a 64 KB tile, as a 512-point line's), longer lines than
-// 128-byte rows hold take 64- or 32-byte rows with runtime plans.
+// take 64-byte rows (a 64 KB tile, as a 512-point line's).
 #define FF_FOR_EACH_STRIDED_N(X) X(64) X(128) X(256) X(512)
-template <typename T> static StridedKernel<T> strided_kernel(int kind, int N, int W = 128 / (2 * (int)sizeof(T))) {
+template <typename T> static StridedKernel<T> strided_kernel(int kind, int N) {
   constexpr int WF = 128 / (2 * (int)sizeof(T));
-  if (W == WF / 2) return N == 1024 ? strided_nw<T, 1024, WF / 2>(kind) : strided_nw<T, 0, WF / 2>(kind);
-  if (W == WF / 4) return strided_nw<T, 0, WF / 4>(kind);
+  if (N == 1024) return strided_nw<T, 1024, WF / 2>(kind);
 #define FF_CASE(NN) if (N == NN) return strided_nw<T, NN, WF>(kind);
   FF_FOR_EACH_STRIDED_N(FF_CASE)
 #undef FF_CASE
-  return strided_nw<T, 0, WF>(kind);
+  return nullptr;
 }
 
 // (z, y) length pairs with specialised fused kernels; others use (0, 0).
@@ -487,18 +482,13 @@ template <typename T> static int configure(ff_plan *p) {
   p->zsmem = a_bytes + (zfuse ? a_bytes : (size_t)p->zW * p->zP * csz) + 128 + 128;
   const long npairs = ((long)ni * nj + 1) / 2;
   p->ztiles = (unsigned)((npairs + p->zW - 1) / p->zW);
-  // line blocks by bulk copies: whole 16-byte multiples, and a first stage
-  // that is not the last (the bulk-fed tiles stage their input in the buffer
-  // the last stage writes)
-  p->zbulk = p->zN > 0 || ((nk * sizeof(T)) % 16 == 0 && plan_stages(nk) >= 2);
-  if (!p->bsM[2]) {
-    rc = allow_dyn_smem(zfwd_kernel<T>(p->zN, p->zbulk), nullptr);
-    if (rc == FF_OK) rc = allow_dyn_smem(zinv_kernel<T>(p->zN, p->zbulk), nullptr);
+  if (p->zN) {
+    rc = allow_dyn_smem(zfwd_kernel<T>(p->zN), nullptr);
+    if (rc == FF_OK) rc = allow_dyn_smem(zinv_kernel<T>(p->zN), nullptr);
     if (rc != FF_OK) return rc;
   }
-  // strided tiles: W columns of 128-byte rows x n rows, one per block; lines
-  // too long for that (above about 1800 points FP64, 3600 FP32) take 64- or
-  // 32-byte rows, i.e. half or a quarter of the columns per tile
+  // strided tiles: W columns of 128-byte rows x n rows, one per block.  (Of the
+  // lengths without a compile-time plan only the fused passes read this.)
   const int W = 128 / (int)csz;
   for (int kind = 0; kind < 3; kind++) {
     StridedCfg &cfg = kind == 2 ? p->xcfg : p->ycfg;
@@ -511,26 +501,59 @@ template <typename T> static int configure(ff_plan *p) {
     // for a 1024-row tile split over a 2-block cluster and 1.06 ms for one
     // block of 128-byte rows per SM)
     if (cfg.N == 1024) cfg.W = W / 2;
-    while ((size_t)n * cfg.W * csz + 1024 > kMaxDynSmem && cfg.W * csz > 32) {
-      cfg.W /= 2;
-      cfg.N = 0;
-    }
+    while ((size_t)n * cfg.W * csz + 1024 > kMaxDynSmem && cfg.W * csz > 32) cfg.W /= 2;
     cfg.box_rows = largest_divisor_at_most(n, 256, 1);
     cfg.smem = (size_t)n * cfg.W * csz + 128;
-    size_t avail = 0;
-    rc = allow_dyn_smem(strided_kernel<T>(kind, cfg.N, cfg.W), &avail);
-    if (rc != FF_OK) return rc;
-    if (cfg.smem > avail) return set_error(FF_ERR_UNSUPPORTED, "no tile shape for an axis of %d points", n);
+    if (cfg.N) {
+      size_t avail = 0;
+      rc = allow_dyn_smem(strided_kernel<T>(kind, cfg.N), &avail);
+      if (rc != FF_OK) return rc;
+      if (cfg.smem > avail) return set_error(FF_ERR_UNSUPPORTED, "no tile shape for an axis of %d points", n);
+    }
     cfg.grid = (kind == 2 ? nj : ni) * ((p->nh + cfg.W - 1) / cfg.W);
+  }
+  // lengths without a compile-time plan
+  for (int d = 0; d < 3; d++) {
+    if (!p->gen[d]) continue;
+    const int kind = d == 2 ? 0 : d == 1 ? 1 : 2;
+    const std::vector<int> radix = gen_radices(p->n[d], d == 2);
+    p->gshape[d] = gen_shape(kind, ni, nj, nk, p->nhp, (int)sizeof(T), radix, p->num_sms);
+    const GenShape &sh = p->gshape[d];
+    for (int k = kind; k <= 4 && rc == FF_OK; k = k == 0 ? 4 : k == 1 ? 3 : 5) rc = gen_prepare<T>(k, sh.smem);
+    if (rc != FF_OK) return rc;
+    auto fill = [&](auto &g) {
+      gen_stages(p->n[d], radix, d == 2 ? gen_pad(nk, radix) : 0, sh.threads, sh.units, &g.ax.S, g.ax.st);
+      g.ni = ni;
+      g.nj = nj;
+      g.nk = nk;
+      g.nh = p->nh;
+      g.nhp = p->nhp;
+      for (g.lu = 0; (1 << g.lu) < sh.units;) g.lu++;
+      g.box_rows = sh.box_rows;
+      g.tile_rows = sh.tile_rows;
+      g.lp = sh.lp;
+      g.sp = sh.sp;
+      g.per_line = (nk * sizeof(T)) % 16 == 0;
+      for (int q = 0; q < 3; q++) g.dd[q] = p->dd[q];
+      g.invN = 1.0 / (double(ni) * double(nj) * double(nk));
+      g.status = p->status;
+      g.wait_iters = 0;
+      // the resident blocks' successors (as the compile-time z passes do)
+      const int per_sm = std::max(1, std::min((int)(kMaxDynSmem / (sh.smem + 1024)), 768 / sh.threads));
+      g.l2_ahead = per_sm * p->num_sms;
+    };
+    if constexpr (sizeof(T) == 8) fill(p->gpd[d]);
+    else fill(p->gpf[d]);
   }
   const int ktiles = (p->nh + W - 1) / W;
   // the fused passes hold a whole y tile of 128-byte rows per block (not with
   // Bluestein axes or narrowed tiles)
-  const bool can_fuse = !any_bs && p->ycfg.W == W && p->xcfg.W == W;
+  const char *mode = getenv("FF_PASSES");
+  p->fused = mode && strcmp(mode, "3") == 0 && !any_bs && p->ycfg.W == W && p->xcfg.W == W;
   // fused passes: persistent blocks over the in-order tile queue (not with
   // Bluestein axes)
   const int zpp = (nj + 2 * p->zW - 1) / (2 * p->zW);   // z tiles per plane (pairs never cross planes)
-  for (int dir = 0; dir < 2 && can_fuse; dir++) {
+  for (int dir = 0; dir < 2 && p->fused; dir++) {
     FusedCfg &fc = dir == 0 ? p->fwd : p->inv;
     fused_pair(nk, nj, &fc.NZ, &fc.NY);
     fc.smem = std::max(p->zsmem, p->ycfg.smem);
@@ -566,8 +589,6 @@ template <typename T> static int configure(ff_plan *p) {
   // L2.  (The same hint on the strided passes' tensor tiles slowed them.)
   const char *ahead = getenv("FF_L2_AHEAD");
   p->l2_ahead = ahead ? std::max(0, atoi(ahead)) : 6 * p->num_sms;
-  const char *mode = getenv("FF_PASSES");
-  p->fused = mode && strcmp(mode, "3") == 0 && can_fuse;
   return FF_OK;
 }
 
@@ -609,9 +630,50 @@ int encode_spectrum_map(void *base, int ni, int nj, int nh, int nhp, size_t esz,
   return FF_OK;
 }
 
-template <typename T> static int spectrum_map(const ff_plan *p, void *base, const StridedCfg &cfg, bool xpass,
-                                              CUtensorMap *map) {
-  return encode_spectrum_map(base, p->n[0], p->n[1], p->nh, p->nhp, sizeof(T), cfg.W, cfg.box_rows, xpass, map);
+// Tensor map of the y (axis 1) or x (axis 0) pass on the half spectrum at base.
+template <typename T> static int spectrum_map(const ff_plan *p, void *base, int axis, bool fused, CUtensorMap *map) {
+  const StridedCfg &cfg = axis == 0 ? p->xcfg : p->ycfg;
+  int W = cfg.W, rows = cfg.box_rows;
+  if (p->gen[axis] && !fused) {
+    W = p->gshape[axis].units * 16 / (2 * (int)sizeof(T));
+    rows = p->gshape[axis].box_rows;
+  }
+  return encode_spectrum_map(base, p->n[0], p->n[1], p->nh, p->nhp, sizeof(T), W, rows, axis == 0, map);
+}
+
+// One y or x pass (kind 1 y forward, 2 x, 3 y inverse) through the generic or
+// the compile-time kernels.
+template <typename T>
+static int launch_strided(const ff_plan *p, int kind, const CUtensorMap &map, typename Cplx<T>::type *dst,
+                          const PassArgs<T> &a, cudaStream_t st) {
+  const int axis = kind == 2 ? 0 : 1;
+  if (p->gen[axis]) return gen_launch<T>(kind, gen_pass<T>(p, axis), p->gshape[axis], &map, nullptr, dst, st);
+  const StridedCfg &cfg = axis == 0 ? p->xcfg : p->ycfg;
+  strided_kernel<T>(kind == 1 ? 0 : kind == 3 ? 1 : 2, cfg.N)<<<cfg.grid, kZThreads, cfg.smem, st>>>(
+      map, dst, a, cfg.box_rows);
+  FF_CUDA(cudaGetLastError());
+  return FF_OK;
+}
+
+template <typename T> static int launch_z(const ff_plan *p, bool inverse, void *in, void *out, cudaStream_t st) {
+  using C = typename Cplx<T>::type;
+  const PassArgs<T> a = pass_args<T>(p);
+  if (p->bsM[2]) {
+    const BsAxis<C> *bs;
+    if constexpr (sizeof(T) == 8) bs = &p->bsd[2];
+    else bs = &p->bsf[2];
+    return bs_launch<T>(inverse ? 4 : 0, in, out, a, *bs, p->bscfg[inverse ? 4 : 0], st);
+  }
+  if (p->gen[2])
+    return gen_launch<T>(inverse ? 4 : 0, gen_pass<T>(p, 2), p->gshape[2], nullptr, in, out, st);
+  if (!inverse)
+    zfwd_kernel<T>(p->zN)<<<p->ztiles, kZPassThreads, p->zsmem, st>>>(static_cast<const T *>(in),
+                                                                          static_cast<C *>(out), a, p->zW, p->zP);
+  else
+    zinv_kernel<T>(p->zN)<<<p->ztiles, kZPassThreads, p->zsmem, st>>>(static_cast<const C *>(in),
+                                                                          static_cast<T *>(out), a, p->zW, p->zP);
+  FF_CUDA(cudaGetLastError());
+  return FF_OK;
 }
 
 template <typename T>
@@ -625,8 +687,8 @@ static int launch_solve(const ff_plan *p, void *density, void *potential, cudaSt
   C *Ps = reinterpret_cast<C *>(potential);
   CUtensorMap ymapP, xmapP;
   int rc = FF_OK;
-  if (!p->bsM[1]) rc = spectrum_map<T>(p, potential, p->ycfg, false, &ymapP);
-  if (rc == FF_OK && !p->bsM[0]) rc = spectrum_map<T>(p, potential, p->xcfg, true, &xmapP);
+  if (!p->bsM[1]) rc = spectrum_map<T>(p, potential, 1, p->fused, &ymapP);
+  if (rc == FF_OK && !p->bsM[0]) rc = spectrum_map<T>(p, potential, 0, false, &xmapP);
   if (rc != FF_OK) return rc;
   auto bsax = [&](int d) -> const BsAxis<C> & {
     if constexpr (sizeof(T) == 8) return p->bsd[d];
@@ -642,8 +704,8 @@ static int launch_solve(const ff_plan *p, void *density, void *potential, cudaSt
     fwd_kernel<T>(p->fwd.NZ, p->fwd.NY)<<<p->fwd.grid, kZThreads, p->fwd.smem, st>>>(D, Ps, a, ff);
     FF_CUDA(cudaGetLastError());
     if (timed) FF_CUDA(cudaEventRecord(p->ev[ev++], st));
-    strided_kernel<T>(2, p->xcfg.N, p->xcfg.W)<<<p->xcfg.grid, kZThreads, p->xcfg.smem, st>>>(xmapP, Ps, a, p->xcfg.box_rows);
-    FF_CUDA(cudaGetLastError());
+    rc = launch_strided<T>(p, 2, xmapP, Ps, a, st);
+    if (rc != FF_OK) return rc;
     if (timed) FF_CUDA(cudaEventRecord(p->ev[ev++], st));
     FuseArgs fi{p->counters + 1, p->counters + 2 + ni, ni, p->inv.prod_pp, p->inv.cons_pp, p->inv.lag, p->zW, p->zP,
                 p->ycfg.box_rows, p->wait_iters, p->dep_extra};
@@ -653,21 +715,16 @@ static int launch_solve(const ff_plan *p, void *density, void *potential, cudaSt
     return FF_OK;
   }
   // each pass through the Bluestein kernels where its axis needs them
-  if (p->bsM[2]) {
-    rc = bs_launch<T>(0, D, Ps, a, bsax(2), p->bscfg[0], st);
-    if (rc != FF_OK) return rc;
-  } else {
-    zfwd_kernel<T>(p->zN, p->zbulk)<<<p->ztiles, kZPassThreads, p->zsmem, st>>>(D, Ps, a, p->zW, p->zP);
-    FF_CUDA(cudaGetLastError());
-  }
+  rc = launch_z<T>(p, false, D, Ps, st);
+  if (rc != FF_OK) return rc;
   if (timed) FF_CUDA(cudaEventRecord(p->ev[ev++], st));
   if (npass == 1) return FF_OK;
   if (p->bsM[1]) {
     rc = bs_launch<T>(1, Ps, Ps, a, bsax(1), p->bscfg[1], st);
     if (rc != FF_OK) return rc;
   } else {
-    strided_kernel<T>(0, p->ycfg.N, p->ycfg.W)<<<p->ycfg.grid, kZThreads, p->ycfg.smem, st>>>(ymapP, Ps, a, p->ycfg.box_rows);
-    FF_CUDA(cudaGetLastError());
+    rc = launch_strided<T>(p, 1, ymapP, Ps, a, st);
+    if (rc != FF_OK) return rc;
   }
   if (timed) FF_CUDA(cudaEventRecord(p->ev[ev++], st));
   if (npass == 2) return FF_OK;
@@ -675,8 +732,8 @@ static int launch_solve(const ff_plan *p, void *density, void *potential, cudaSt
     rc = bs_launch<T>(2, Ps, Ps, a, bsax(0), p->bscfg[2], st);
     if (rc != FF_OK) return rc;
   } else {
-    strided_kernel<T>(2, p->xcfg.N, p->xcfg.W)<<<p->xcfg.grid, kZThreads, p->xcfg.smem, st>>>(xmapP, Ps, a, p->xcfg.box_rows);
-    FF_CUDA(cudaGetLastError());
+    rc = launch_strided<T>(p, 2, xmapP, Ps, a, st);
+    if (rc != FF_OK) return rc;
   }
   if (timed) FF_CUDA(cudaEventRecord(p->ev[ev++], st));
   if (npass == 3) return FF_OK;
@@ -684,18 +741,13 @@ static int launch_solve(const ff_plan *p, void *density, void *potential, cudaSt
     rc = bs_launch<T>(3, Ps, Ds, a, bsax(1), p->bscfg[3], st);
     if (rc != FF_OK) return rc;
   } else {
-    strided_kernel<T>(1, p->ycfg.N, p->ycfg.W)<<<p->ycfg.grid, kZThreads, p->ycfg.smem, st>>>(ymapP, Ds, a, p->ycfg.box_rows);
-    FF_CUDA(cudaGetLastError());
+    rc = launch_strided<T>(p, 3, ymapP, Ds, a, st);
+    if (rc != FF_OK) return rc;
   }
   if (timed) FF_CUDA(cudaEventRecord(p->ev[ev++], st));
   if (npass == 4) return FF_OK;
-  if (p->bsM[2]) {
-    rc = bs_launch<T>(4, Ds, P, a, bsax(2), p->bscfg[4], st);
-    if (rc != FF_OK) return rc;
-  } else {
-    zinv_kernel<T>(p->zN, p->zbulk)<<<p->ztiles, kZPassThreads, p->zsmem, st>>>(Ds, P, a, p->zW, p->zP);
-    FF_CUDA(cudaGetLastError());
-  }
+  rc = launch_z<T>(p, true, Ds, P, st);
+  if (rc != FF_OK) return rc;
   if (timed) FF_CUDA(cudaEventRecord(p->ev[ev++], st));
   return FF_OK;
 }
@@ -706,25 +758,6 @@ int allow_dyn_smem_fn(const void *fn, size_t *avail) {
   const size_t lim = kMaxDynSmem - fa.sharedSizeBytes;
   FF_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim));
   if (avail) *avail = lim;
-  return FF_OK;
-}
-
-template <typename T> static int launch_z(const ff_plan *p, bool inverse, void *in, void *out, cudaStream_t st) {
-  using C = typename Cplx<T>::type;
-  const PassArgs<T> a = pass_args<T>(p);
-  if (p->bsM[2]) {
-    const BsAxis<C> *bs;
-    if constexpr (sizeof(T) == 8) bs = &p->bsd[2];
-    else bs = &p->bsf[2];
-    return bs_launch<T>(inverse ? 4 : 0, in, out, a, *bs, p->bscfg[inverse ? 4 : 0], st);
-  }
-  if (!inverse)
-    zfwd_kernel<T>(p->zN, p->zbulk)<<<p->ztiles, kZPassThreads, p->zsmem, st>>>(static_cast<const T *>(in),
-                                                                          static_cast<C *>(out), a, p->zW, p->zP);
-  else
-    zinv_kernel<T>(p->zN, p->zbulk)<<<p->ztiles, kZPassThreads, p->zsmem, st>>>(static_cast<const C *>(in),
-                                                                          static_cast<T *>(out), a, p->zW, p->zP);
-  FF_CUDA(cudaGetLastError());
   return FF_OK;
 }
 
@@ -841,14 +874,29 @@ int ff_plan_create(const int n[3], const double lo[3], const double hi[3], int p
     rev[d] = plan_digit_reversal(L, radix[d]);
     o_tw[d] = take(L * csz);
     o_tw64[d] = precision == FF_FP64 ? o_tw[d] : take(L * sizeof(double2));
-    o_rev[d] = take(L * sizeof(int));
-    o_ipos[d] = take(L * sizeof(int));
     o_kk[d] = take((d == 2 ? p->nh : n[d]) * sizeof(double));
     if (p->bsM[d]) {
       o_chirp[d] = take(n[d] * csz);
       o_ghat[d] = take(L * csz);
     }
   }
+  size_t o_gen[3] = {0, 0, 0}, o_gidx[3] = {0, 0, 0};
+  std::vector<int> gradix[3], gidx[3];
+  for (int d = 0; d < 3; d++) {
+    p->gen[d] = !p->bsM[d] && special_n(n[d]) == 0;
+    if (!p->gen[d]) continue;
+    gradix[d] = gen_radices(n[d], d == 2);
+    o_gen[d] = take(gen_axis_bytes(n[d], (int)csz / 2));
+    gen_index(n[d], gradix[d], d == 2 ? gen_pad(n[d], gradix[d]) : 0, d == 2, &gidx[d]);
+  }
+  // the integer tables, one upload
+  const size_t o_int = off;
+  for (int d = 0; d < 3; d++) {
+    o_rev[d] = take(len[d] * sizeof(int));
+    o_ipos[d] = take(len[d] * sizeof(int));
+    if (p->gen[d]) o_gidx[d] = take(gidx[d].size() * sizeof(int));
+  }
+  const size_t int_bytes = off - o_int;
   const size_t o_status = take(sizeof(int));
   const size_t o_counters = take((2 + 2 * (size_t)n[0]) * sizeof(int));
   for (int e = 0; e <= FF_MAX_PHASES; e++) {
@@ -869,13 +917,22 @@ int ff_plan_create(const int n[3], const double lo[3], const double hi[3], int p
   p->counters = reinterpret_cast<int *>(base + o_counters);
   int rc = FF_OK;
   if (cudaMemset(p->status, 0, sizeof(int)) != cudaSuccess) rc = set_error(FF_ERR_CUDA, "ff_plan_create: memset");
+  {
+    std::vector<char> host(int_bytes, 0);
+    for (int d = 0; d < 3; d++) {
+      int *hrev = reinterpret_cast<int *>(host.data() + (o_rev[d] - o_int));
+      int *hpos = reinterpret_cast<int *>(host.data() + (o_ipos[d] - o_int));
+      for (int q = 0; q < len[d]; q++) {
+        hrev[q] = rev[d][q];
+        hpos[rev[d][q]] = q;
+      }
+      if (p->gen[d]) std::memcpy(host.data() + (o_gidx[d] - o_int), gidx[d].data(), gidx[d].size() * sizeof(int));
+    }
+    if (rc == FF_OK && cudaMemcpy(base + o_int, host.data(), int_bytes, cudaMemcpyHostToDevice) != cudaSuccess)
+      rc = set_error(FF_ERR_CUDA, "ff_plan_create: table upload failed");
+  }
   for (int d = 0; d < 3 && rc == FF_OK; d++) {
     const int L = len[d];
-    std::vector<int> ipos(L);
-    for (int q = 0; q < L; q++) ipos[rev[d][q]] = q;
-    if (cudaMemcpy(base + o_rev[d], rev[d].data(), L * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(base + o_ipos[d], ipos.data(), L * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
-      rc = set_error(FF_ERR_CUDA, "ff_plan_create: table upload failed");
     const int blocks = std::min(1024, (L + 255) / 256);
     k_twiddles<<<blocks, 256>>>(L, reinterpret_cast<double2 *>(base + o_tw64[d]));
     if (precision == FF_FP32) k_twiddles<<<blocks, 256>>>(L, reinterpret_cast<float2 *>(base + o_tw[d]));
@@ -895,6 +952,11 @@ int ff_plan_create(const int n[3], const double lo[3], const double hi[3], int p
     ad.ipos = af.ipos = reinterpret_cast<const int *>(base + o_ipos[d]);
     p->axd[d] = ad;
     p->axf[d] = af;
+    if (p->gen[d] && rc == FF_OK) {
+      const int *idx = reinterpret_cast<const int *>(base + o_gidx[d]);
+      rc = precision == FF_FP64 ? gen_axis_build(n[d], gradix[d], base + o_gen[d], idx, &p->gpd[d].ax)
+                                : gen_axis_build(n[d], gradix[d], base + o_gen[d], idx, &p->gpf[d].ax);
+    }
     if (p->bsM[d] && rc == FF_OK) {
       const int *drev = reinterpret_cast<const int *>(base + o_rev[d]);
       if (precision == FF_FP64) {
