@@ -7,7 +7,7 @@
 // c[j] = exp(-i*pi*j^2/n), the forward DFT is
 //   X[k] = c[k] * sum_j (x[j] c[j]) conj c[k-j],
 // a circular convolution of M >= 2n-1 points (M = 2^a 3^b 5^c 7^d), computed by
-// the same mixed-radix stages as every other axis: an M-point forward DIF
+// the stages of the generic passes (ff_gen_stages.cuh): an M-point forward DIF
 // transform of the premultiplied, zero-padded line, a product with the
 // transform of the convolution kernel (one register group, with the last DIF
 // and first DIT stages), an M-point inverse DIT transform, and the
@@ -20,46 +20,44 @@
 
 #include <cuda_runtime.h>
 
-#include "ff_tiles.cuh"
+#include <vector>
+
+#include "ff_gen.hpp"
 
 namespace ff {
 
-template <typename C> struct BsAxis {
-  AxisDev<C> m;      // plan and twiddle tables of the M-point transforms
+// Pass arguments: those of the generic passes, whose axis is the M-point
+// transform, and
+template <typename C> struct BsPass : GenPass<C> {
   int n;             // axis length
   const C *chirp;    // chirp[j] = exp(-i*pi*j^2/n), j < n (FP64-generated)
   const C *ghat;     // ghat[pos] = G[k]/M for the frequency k at DIF output position pos,
                      // G the M-point DFT of g[m] = conj chirp[|m|] (|m| < n, indices mod M)
 };
 
-// Smallest 2^a 3^b 5^c 7^d >= 2n - 1.
+// The transform length M of an axis of n points.
 int bs_padded_length(int n);
 
-// Launch shape of one Bluestein pass.
-struct BsCfg {
-  int W;          // z: line pairs per block; y, x: columns per tile
-  int P;          // z: line pitch in complex values (multiple of 8 FP64 / 16 FP32)
-  size_t smem;    // dynamic shared memory per block
-  long grid;      // blocks
-};
+// Launch shape of pass `kind` (0 z forward, 1 y forward, 2 x, 3 y inverse,
+// 4 z inverse) of an ni x nj x nk grid whose axis for that pass goes through
+// M points.
+GenShape bs_shape(int kind, int ni, int nj, int nk, int nhp, int esz, int M, int num_sms);
 
-// Chooses the launch shape of pass `kind` (0 z forward, 1 y forward, 2 x,
-// 3 y inverse, 4 z inverse) of an ni x nj x nk plan whose axis for that pass
-// is transformed through M points, and raises the kernel's shared-memory
-// limit.  FF_OK or an FF_ERR_* status.
-template <typename T> int bs_configure(int kind, int ni, int nj, int nh, int M, BsCfg *cfg);
+// Raises the pass kernel's shared-memory limit; FF_ERR_UNSUPPORTED if the tile
+// does not fit.
+template <typename T> int bs_prepare(int kind, size_t smem);
 
 // Device tables of one axis: chirp (n values) and ghat (M values, from the
-// M-point plan's digit reversal rev).  Enqueued on the current device's
-// default stream.
-template <typename C> int bs_tables(int n, int M, const int *rev, C *chirp, C *ghat);
+// M-point plan's group bases k0 and last radix).  Enqueued on the current
+// device's default stream.
+template <typename C> int bs_tables(int n, int M, const int *k0, int last_radix, C *chirp, C *ghat);
 
-// Pass launches (kind numbering as in bs_configure).  src and dst are the
-// pass's input and output arrays as the regular passes use them: z forward
-// reads the real field and writes the spectrum; y forward and x work in place
-// on the spectrum; y inverse reads one spectrum array and writes the other;
-// z inverse reads the spectrum and writes the real field.
-template <typename T> int bs_launch(int kind, const void *src, void *dst, const PassArgs<T> &a,
-                                    const BsAxis<typename Cplx<T>::type> &bs, const BsCfg &cfg, cudaStream_t st);
+// Pass launches.  in and out are the pass's arrays as the regular passes use
+// them: z forward reads the real field and writes the spectrum; y forward and
+// x work in place on the spectrum; y inverse reads one spectrum array and
+// writes the other; z inverse reads the spectrum and writes the real field.
+template <typename T>
+int bs_launch(int kind, const BsPass<typename Cplx<T>::type> &a, const GenShape &s, const void *in, void *out,
+              cudaStream_t st);
 
 }  // namespace ff

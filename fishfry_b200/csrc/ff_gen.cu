@@ -81,6 +81,13 @@ std::vector<int> gen_bases(int n, const std::vector<int> &radix) {
   return k0;
 }
 
+double gen_cost(int n) {
+  const std::vector<int> r = gen_radices(n, false);
+  double c = 0.0;
+  for (size_t s = 0; s < r.size(); s++) c += stage_cost(r[s], s + 1 == r.size());
+  return c;
+}
+
 int gen_pad(int n, const std::vector<int> &radix) { return radix.size() > 1 && (n / radix[0]) % 2 == 0 ? 1 : 0; }
 
 int gen_table_size(int n, const std::vector<int> &radix) {
@@ -183,42 +190,46 @@ constexpr size_t kSmSmem = 227 * 1024;
 // Smallest v >= lo with v = rem mod step.
 int next_congruent(int lo, int rem, int step) { return lo + ((rem - lo) % step + step) % step; }
 
-// Threads per block: 24 warps on an SM at the tile's shared memory (80
-// registers a thread).
-int pick_threads(size_t smem) {
-  const int blocks = (int)std::max<size_t>(1, std::min<size_t>(8, kSmSmem / (smem + 1024)));
-  return std::min(256, std::max(64, 768 / blocks / 32 * 32));
+}  // namespace
+
+// 24 warps on an SM at the tile's shared memory (80 registers a thread).
+void gen_pick_threads(GenShape *s) {
+  const int blocks = (int)std::max<size_t>(1, std::min<size_t>(8, kSmSmem / (s->smem + 1024)));
+  s->threads = std::min(256, std::max(64, 768 / blocks / 32 * 32));
 }
 
-}  // namespace
+void gen_z_shape(GenShape *s, int ni, int nj, int nk, int nhp, int esz, int num_sms) {
+  const int cu = 16 / (2 * esz);   // line pairs per unit
+  const long nlines = (long)ni * nj;
+  // many small tiles (up to 40 KB, five or more blocks on an SM) beat fewer
+  // large ones for short lines and tie for long ones: 200x180x160 FP32 z
+  // 20.9 / 21.5 us against 26.2 / 23.5 at 56 KB, 500^3 FP64 425 / 431 against
+  // 443 / 455 at 74 KB
+  const size_t limit = 40 * 1024;
+  for (s->units = 8;; s->units /= 2) {
+    const int lines = 2 * cu * s->units;
+    // pitches that put neighbouring units' lines and rows in different banks
+    const bool per_line = (nk * esz) % 16 == 0;
+    const int vals = 16 / esz;   // values per 16 bytes
+    s->lp = per_line ? next_congruent(nk, std::max(vals, 64 / esz / s->units) % (64 / esz), 64 / esz) : nk;
+    const int per = 64 / (2 * esz);
+    s->sp = next_congruent(nhp, std::max(cu, per / s->units) % per, per);
+    const size_t tile = ((size_t)s->tile_rows * s->units * 16 + 127) & ~size_t(127);
+    const size_t stage = std::max((size_t)lines * s->lp * esz + 16, (size_t)lines * s->sp * 2 * esz);
+    s->smem = tile + ((stage + 127) & ~size_t(127)) + 128;
+    s->grid = (nlines + lines - 1) / lines;
+    if (s->units == 1) break;
+    if (s->smem <= limit && (s->grid >= num_sms || s->units <= 2)) break;
+  }
+  gen_pick_threads(s);
+}
 
 GenShape gen_shape(int kind, int ni, int nj, int nk, int nhp, int esz, const std::vector<int> &radix, int num_sms) {
   GenShape s{};
   const int cu = 16 / (2 * esz);   // complex columns (or line pairs) per unit
   if (kind == 0 || kind == 4) {
-    const long nlines = (long)ni * nj;
-    // many small tiles (up to 40 KB, five or more blocks on an SM) beat fewer
-    // large ones for short lines and tie for long ones: 200x180x160 FP32 z
-    // 20.9 / 21.5 us against 26.2 / 23.5 at 56 KB, 500^3 FP64 425 / 431 against
-    // 443 / 455 at 74 KB
-    const size_t limit = 40 * 1024;
     s.tile_rows = nk + gen_pad(nk, radix) * (radix[0] - 1);
-    for (s.units = 8;; s.units /= 2) {
-      const int lines = 2 * cu * s.units;
-      // pitches that put neighbouring units' lines and rows in different banks
-      const bool per_line = (nk * esz) % 16 == 0;
-      const int vals = 16 / esz;   // values per 16 bytes
-      s.lp = per_line ? next_congruent(nk, std::max(vals, 64 / esz / s.units) % (64 / esz), 64 / esz) : nk;
-      const int per = 64 / (2 * esz);
-      s.sp = next_congruent(nhp, std::max(cu, per / s.units) % per, per);
-      const size_t tile = ((size_t)s.tile_rows * s.units * 16 + 127) & ~size_t(127);
-      const size_t stage = std::max((size_t)lines * s.lp * esz + 16, (size_t)lines * s.sp * 2 * esz);
-      s.smem = tile + ((stage + 127) & ~size_t(127)) + 128;
-      s.grid = (nlines + lines - 1) / lines;
-      if (s.units == 1) break;
-      if (s.smem <= limit && (s.grid >= num_sms || s.units <= 2)) break;
-    }
-    s.threads = pick_threads(s.smem);
+    gen_z_shape(&s, ni, nj, nk, nhp, esz, num_sms);
     return s;
   }
   const int n = kind == 2 ? ni : nj;
@@ -242,7 +253,7 @@ GenShape gen_shape(int kind, int ni, int nj, int nk, int nhp, int esz, const std
     if (s.units == 2) break;
     if (s.units == 8 ? s.smem <= 74 * 1024 && s.grid >= num_sms : s.smem <= kSmSmem - 1024) break;
   }
-  s.threads = pick_threads(s.smem);
+  gen_pick_threads(&s);
   return s;
 }
 

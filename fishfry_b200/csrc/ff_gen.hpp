@@ -77,6 +77,15 @@ struct GenShape {
 // ni x nj x nk grid; esz: bytes of a real value.
 GenShape gen_shape(int kind, int ni, int nj, int nk, int nhp, int esz, const std::vector<int> &radix, int num_sms);
 
+// Parts of gen_shape that other tiles share: units, pitches, shared memory and
+// grid of a z pass whose tile has s->tile_rows rows; threads per block from the
+// shared memory.
+void gen_z_shape(GenShape *s, int ni, int nj, int nk, int nhp, int esz, int num_sms);
+void gen_pick_threads(GenShape *s);
+
+// Cost of an n-point transform's stages per point (arbitrary unit).
+double gen_cost(int n);
+
 // What the pass kernels need besides the axis.
 template <typename C> struct GenPass {
   int ni, nj, nk, nh, nhp;

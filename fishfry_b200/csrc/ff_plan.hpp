@@ -44,7 +44,6 @@ struct ff_plan {
   void *dmem;
   ff::AxisDev<double2> axd[3];
   ff::AxisDev<float2> axf[3];
-  double *kk[3];
   int *status;
   int *counters;       // fused passes: 2 tickets + 2 x ni plane counts
   int fused;           // 1: three launches (fused z/y passes), 0: five launches
@@ -58,14 +57,12 @@ struct ff_plan {
   ff::StridedCfg ycfg, xcfg;
   ff::FusedCfg fwd, inv;
   // axes with a prime factor above 7: padded convolution length M (0 for a
-  // 2^a 3^b 5^c 7^d axis), their tables, and the launch shape of each pass kind
-  // (0 z fwd, 1 y fwd, 2 x, 3 y inv, 4 z inv) that transforms such an axis
+  // 2^a 3^b 5^c 7^d axis), pass arguments and launch shape by axis
   int bsM[3];
-  ff::BsAxis<double2> bsd[3];
-  ff::BsAxis<float2> bsf[3];
-  ff::BsCfg bscfg[5];
+  ff::BsPass<double2> bspd[3];
+  ff::BsPass<float2> bspf[3];
   // axes of 2^a 3^b 5^c 7^d points without a compile-time plan (ff_gen_dev.cuh):
-  // pass arguments and launch shape by axis
+  // pass arguments by axis, and the launch shape of these and the axes above
   bool gen[3];
   ff::GenPass<double2> gpd[3];
   ff::GenPass<float2> gpf[3];
@@ -86,7 +83,7 @@ template <typename T> PassArgs<T> pass_args(const ff_plan *p) {
   for (int d = 0; d < 3; d++) {
     if constexpr (sizeof(T) == 8) a.ax[d] = p->axd[d];
     else a.ax[d] = p->axf[d];
-    a.kk[d] = p->kk[d];
+    a.kk[d] = nullptr;
   }
   a.invN = 1.0 / (double(p->n[0]) * double(p->n[1]) * double(p->n[2]));
   for (int d = 0; d < 3; d++) a.dd[d] = p->dd[d];
@@ -96,18 +93,21 @@ template <typename T> PassArgs<T> pass_args(const ff_plan *p) {
   return a;
 }
 
-// The generic passes' arguments of axis d, and their launch (kind as
-// gen_launch numbers it; st: stream).
+// The generic (or Bluestein) passes' arguments of axis d with the plan's
+// current wait limit.
 template <typename T> GenPass<typename Cplx<T>::type> gen_pass(const ff_plan *p, int d) {
-  if constexpr (sizeof(T) == 8) {
-    GenPass<double2> a = p->gpd[d];
-    a.wait_iters = p->wait_iters;
-    return a;
-  } else {
-    GenPass<float2> a = p->gpf[d];
-    a.wait_iters = p->wait_iters;
-    return a;
-  }
+  GenPass<typename Cplx<T>::type> a;
+  if constexpr (sizeof(T) == 8) a = p->gpd[d];
+  else a = p->gpf[d];
+  a.wait_iters = p->wait_iters;
+  return a;
+}
+template <typename T> BsPass<typename Cplx<T>::type> bs_pass(const ff_plan *p, int d) {
+  BsPass<typename Cplx<T>::type> a;
+  if constexpr (sizeof(T) == 8) a = p->bspd[d];
+  else a = p->bspf[d];
+  a.wait_iters = p->wait_iters;
+  return a;
 }
 
 // Tensor map of a half spectrum at `base` (ni planes of nj rows of nh complex

@@ -299,15 +299,6 @@ static void launch_x(const CUtensorMap &map, typename Cplx<T>::type *dst, const 
   k_strided<T, W, true, false, N><<<grid, kZThreads, smem, st>>>(map, dst, a, box_rows);
 }
 
-// ------------------------------------------------------------- plan tables
-// (min(i, n-i) * dd)^2 in FP64, as ParisPencil.cpp:276-278 (sqr of the scaled index).
-__global__ void k_wavenumbers(int n, int count, int folded, double dd, double *kk) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-    const double x = double(folded ? min(i, n - i) : i) * dd;
-    kk[i] = x * x;
-  }
-}
-
 }  // namespace ff
 
 // ====================================================================== plan
@@ -459,12 +450,6 @@ template <typename T> static int configure(ff_plan *p) {
   const size_t csz = sizeof(C);
   const int ni = p->n[0], nj = p->n[1], nk = p->n[2];
   int rc = FF_OK;
-  // passes along an axis with a prime factor above 7 (pass kind -> axis)
-  const int axis_of_kind[5] = {2, 1, 0, 1, 2};
-  for (int kind = 0; kind < 5 && rc == FF_OK; kind++)
-    if (p->bsM[axis_of_kind[kind]])
-      rc = bs_configure<T>(kind, ni, nj, p->nh, p->bsM[axis_of_kind[kind]], &p->bscfg[kind]);
-  if (rc != FF_OK) return rc;
   const bool any_bs = p->bsM[0] || p->bsM[1] || p->bsM[2];
   // z tiles: W line pairs, two line-major buffers of pitch P, ~32 KB per
   // block of kZPassThreads threads (six blocks per SM)
@@ -512,17 +497,22 @@ template <typename T> static int configure(ff_plan *p) {
     }
     cfg.grid = (kind == 2 ? nj : ni) * ((p->nh + cfg.W - 1) / cfg.W);
   }
-  // lengths without a compile-time plan
+  // lengths without a compile-time plan, and those with a prime factor above 7
   for (int d = 0; d < 3; d++) {
-    if (!p->gen[d]) continue;
+    if (!p->gen[d] && !p->bsM[d]) continue;
     const int kind = d == 2 ? 0 : d == 1 ? 1 : 2;
-    const std::vector<int> radix = gen_radices(p->n[d], d == 2);
-    p->gshape[d] = gen_shape(kind, ni, nj, nk, p->nhp, (int)sizeof(T), radix, p->num_sms);
-    const GenShape &sh = p->gshape[d];
-    for (int k = kind; k <= 4 && rc == FF_OK; k = k == 0 ? 4 : k == 1 ? 3 : 5) rc = gen_prepare<T>(k, sh.smem);
+    const int L = p->gen[d] ? p->n[d] : p->bsM[d];
+    const bool split = p->gen[d] && d == 2;
+    const std::vector<int> radix = gen_radices(L, split);
+    const GenShape sh = p->gen[d]
+        ? gen_shape(kind, ni, nj, nk, p->nhp, (int)sizeof(T), radix, p->num_sms)
+        : bs_shape(kind, ni, nj, nk, p->nhp, (int)sizeof(T), L, p->num_sms);
+    p->gshape[d] = sh;
+    for (int k = kind; k <= 4 && rc == FF_OK; k = k == 0 ? 4 : k == 1 ? 3 : 5)
+      rc = p->gen[d] ? gen_prepare<T>(k, sh.smem) : bs_prepare<T>(k, sh.smem);
     if (rc != FF_OK) return rc;
     auto fill = [&](auto &g) {
-      gen_stages(p->n[d], radix, d == 2 ? gen_pad(nk, radix) : 0, sh.threads, sh.units, &g.ax.S, g.ax.st);
+      gen_stages(L, radix, split ? gen_pad(L, radix) : 0, sh.threads, sh.units, &g.ax.S, g.ax.st);
       g.ni = ni;
       g.nj = nj;
       g.nk = nk;
@@ -542,8 +532,13 @@ template <typename T> static int configure(ff_plan *p) {
       const int per_sm = std::max(1, std::min((int)(kMaxDynSmem / (sh.smem + 1024)), 768 / sh.threads));
       g.l2_ahead = per_sm * p->num_sms;
     };
-    if constexpr (sizeof(T) == 8) fill(p->gpd[d]);
-    else fill(p->gpf[d]);
+    if constexpr (sizeof(T) == 8) {
+      if (p->gen[d]) fill(p->gpd[d]);
+      else fill(p->bspd[d]);
+    } else {
+      if (p->gen[d]) fill(p->gpf[d]);
+      else fill(p->bspf[d]);
+    }
   }
   const int ktiles = (p->nh + W - 1) / W;
   // the fused passes hold a whole y tile of 128-byte rows per block (not with
@@ -641,12 +636,14 @@ template <typename T> static int spectrum_map(const ff_plan *p, void *base, int 
   return encode_spectrum_map(base, p->n[0], p->n[1], p->nh, p->nhp, sizeof(T), W, rows, axis == 0, map);
 }
 
-// One y or x pass (kind 1 y forward, 2 x, 3 y inverse) through the generic or
-// the compile-time kernels.
+// One y or x pass (kind 1 y forward, 2 x, 3 y inverse) through the Bluestein, the
+// generic or the compile-time kernels.  map: the source spectrum src, as the
+// latter two read it.
 template <typename T>
-static int launch_strided(const ff_plan *p, int kind, const CUtensorMap &map, typename Cplx<T>::type *dst,
-                          const PassArgs<T> &a, cudaStream_t st) {
+static int launch_strided(const ff_plan *p, int kind, const CUtensorMap &map, const typename Cplx<T>::type *src,
+                          typename Cplx<T>::type *dst, const PassArgs<T> &a, cudaStream_t st) {
   const int axis = kind == 2 ? 0 : 1;
+  if (p->bsM[axis]) return bs_launch<T>(kind, bs_pass<T>(p, axis), p->gshape[axis], src, dst, st);
   if (p->gen[axis]) return gen_launch<T>(kind, gen_pass<T>(p, axis), p->gshape[axis], &map, nullptr, dst, st);
   const StridedCfg &cfg = axis == 0 ? p->xcfg : p->ycfg;
   strided_kernel<T>(kind == 1 ? 0 : kind == 3 ? 1 : 2, cfg.N)<<<cfg.grid, kZThreads, cfg.smem, st>>>(
@@ -658,12 +655,7 @@ static int launch_strided(const ff_plan *p, int kind, const CUtensorMap &map, ty
 template <typename T> static int launch_z(const ff_plan *p, bool inverse, void *in, void *out, cudaStream_t st) {
   using C = typename Cplx<T>::type;
   const PassArgs<T> a = pass_args<T>(p);
-  if (p->bsM[2]) {
-    const BsAxis<C> *bs;
-    if constexpr (sizeof(T) == 8) bs = &p->bsd[2];
-    else bs = &p->bsf[2];
-    return bs_launch<T>(inverse ? 4 : 0, in, out, a, *bs, p->bscfg[inverse ? 4 : 0], st);
-  }
+  if (p->bsM[2]) return bs_launch<T>(inverse ? 4 : 0, bs_pass<T>(p, 2), p->gshape[2], in, out, st);
   if (p->gen[2])
     return gen_launch<T>(inverse ? 4 : 0, gen_pass<T>(p, 2), p->gshape[2], nullptr, in, out, st);
   if (!inverse)
@@ -690,10 +682,6 @@ static int launch_solve(const ff_plan *p, void *density, void *potential, cudaSt
   if (!p->bsM[1]) rc = spectrum_map<T>(p, potential, 1, p->fused, &ymapP);
   if (rc == FF_OK && !p->bsM[0]) rc = spectrum_map<T>(p, potential, 0, false, &xmapP);
   if (rc != FF_OK) return rc;
-  auto bsax = [&](int d) -> const BsAxis<C> & {
-    if constexpr (sizeof(T) == 8) return p->bsd[d];
-    else return p->bsf[d];
-  };
   int ev = 0;
   if (timed) FF_CUDA(cudaEventRecord(p->ev[ev++], st));
   if (p->fused) {
@@ -704,7 +692,7 @@ static int launch_solve(const ff_plan *p, void *density, void *potential, cudaSt
     fwd_kernel<T>(p->fwd.NZ, p->fwd.NY)<<<p->fwd.grid, kZThreads, p->fwd.smem, st>>>(D, Ps, a, ff);
     FF_CUDA(cudaGetLastError());
     if (timed) FF_CUDA(cudaEventRecord(p->ev[ev++], st));
-    rc = launch_strided<T>(p, 2, xmapP, Ps, a, st);
+    rc = launch_strided<T>(p, 2, xmapP, Ps, Ps, a, st);
     if (rc != FF_OK) return rc;
     if (timed) FF_CUDA(cudaEventRecord(p->ev[ev++], st));
     FuseArgs fi{p->counters + 1, p->counters + 2 + ni, ni, p->inv.prod_pp, p->inv.cons_pp, p->inv.lag, p->zW, p->zP,
@@ -719,31 +707,16 @@ static int launch_solve(const ff_plan *p, void *density, void *potential, cudaSt
   if (rc != FF_OK) return rc;
   if (timed) FF_CUDA(cudaEventRecord(p->ev[ev++], st));
   if (npass == 1) return FF_OK;
-  if (p->bsM[1]) {
-    rc = bs_launch<T>(1, Ps, Ps, a, bsax(1), p->bscfg[1], st);
-    if (rc != FF_OK) return rc;
-  } else {
-    rc = launch_strided<T>(p, 1, ymapP, Ps, a, st);
-    if (rc != FF_OK) return rc;
-  }
+  rc = launch_strided<T>(p, 1, ymapP, Ps, Ps, a, st);
+  if (rc != FF_OK) return rc;
   if (timed) FF_CUDA(cudaEventRecord(p->ev[ev++], st));
   if (npass == 2) return FF_OK;
-  if (p->bsM[0]) {
-    rc = bs_launch<T>(2, Ps, Ps, a, bsax(0), p->bscfg[2], st);
-    if (rc != FF_OK) return rc;
-  } else {
-    rc = launch_strided<T>(p, 2, xmapP, Ps, a, st);
-    if (rc != FF_OK) return rc;
-  }
+  rc = launch_strided<T>(p, 2, xmapP, Ps, Ps, a, st);
+  if (rc != FF_OK) return rc;
   if (timed) FF_CUDA(cudaEventRecord(p->ev[ev++], st));
   if (npass == 3) return FF_OK;
-  if (p->bsM[1]) {
-    rc = bs_launch<T>(3, Ps, Ds, a, bsax(1), p->bscfg[3], st);
-    if (rc != FF_OK) return rc;
-  } else {
-    rc = launch_strided<T>(p, 3, ymapP, Ds, a, st);
-    if (rc != FF_OK) return rc;
-  }
+  rc = launch_strided<T>(p, 3, ymapP, Ps, Ds, a, st);
+  if (rc != FF_OK) return rc;
   if (timed) FF_CUDA(cudaEventRecord(p->ev[ev++], st));
   if (npass == 4) return FF_OK;
   rc = launch_z<T>(p, true, Ds, P, st);
@@ -854,18 +827,23 @@ int ff_plan_create(const int n[3], const double lo[3], const double hi[3], int p
     return set_error(FF_ERR_CUDA, "ff_plan_create: no current CUDA device");
   }
 
-  // device tables: per axis tw (L complex), rev and ipos (L ints) of the
-  // axis's transform length L (n, or the padded M of a Bluestein axis), the
-  // chirp (n) and kernel transform (M) of a Bluestein axis; kk per axis; one
-  // status word
+  // device tables: per axis tw (n complex), rev and ipos (n ints) of the
+  // compile-time and the fused passes; twiddles and an index of the generic
+  // passes' transform (n points, or M of a Bluestein axis); chirp (n) and
+  // kernel transform (M) of a Bluestein axis; one status word
   std::vector<int> radix[3], rev[3];
   int len[3];
   size_t off = 0;
-  size_t o_tw[3], o_tw64[3], o_rev[3], o_ipos[3], o_kk[3], o_chirp[3] = {0, 0, 0}, o_ghat[3] = {0, 0, 0};
+  size_t o_tw[3], o_tw64[3], o_rev[3], o_ipos[3], o_chirp[3] = {0, 0, 0}, o_ghat[3] = {0, 0, 0};
   auto take = [&](size_t b) { size_t o = off; off += (b + 255) & ~size_t(255); return o; };
   for (int d = 0; d < 3; d++) {
     p->bsM[d] = smooth2357(n[d]) ? 0 : bs_padded_length(n[d]);
     const int L = len[d] = p->bsM[d] ? p->bsM[d] : n[d];
+    if (p->bsM[d]) {
+      o_chirp[d] = take(n[d] * csz);
+      o_ghat[d] = take(L * csz);
+      continue;
+    }
     radix[d] = plan_factor_radices(L);
     if ((int)radix[d].size() > kMaxStages) {
       delete p;
@@ -874,27 +852,23 @@ int ff_plan_create(const int n[3], const double lo[3], const double hi[3], int p
     rev[d] = plan_digit_reversal(L, radix[d]);
     o_tw[d] = take(L * csz);
     o_tw64[d] = precision == FF_FP64 ? o_tw[d] : take(L * sizeof(double2));
-    o_kk[d] = take((d == 2 ? p->nh : n[d]) * sizeof(double));
-    if (p->bsM[d]) {
-      o_chirp[d] = take(n[d] * csz);
-      o_ghat[d] = take(L * csz);
-    }
   }
   size_t o_gen[3] = {0, 0, 0}, o_gidx[3] = {0, 0, 0};
   std::vector<int> gradix[3], gidx[3];
   for (int d = 0; d < 3; d++) {
     p->gen[d] = !p->bsM[d] && special_n(n[d]) == 0;
-    if (!p->gen[d]) continue;
-    gradix[d] = gen_radices(n[d], d == 2);
-    o_gen[d] = take(gen_axis_bytes(n[d], (int)csz / 2));
-    gen_index(n[d], gradix[d], d == 2 ? gen_pad(n[d], gradix[d]) : 0, d == 2, &gidx[d]);
+    if (!p->gen[d] && !p->bsM[d]) continue;
+    const bool split = p->gen[d] && d == 2;
+    gradix[d] = gen_radices(len[d], split);
+    o_gen[d] = take(gen_axis_bytes(len[d], (int)csz / 2));
+    gen_index(len[d], gradix[d], split ? gen_pad(len[d], gradix[d]) : 0, split, &gidx[d]);
   }
   // the integer tables, one upload
   const size_t o_int = off;
   for (int d = 0; d < 3; d++) {
-    o_rev[d] = take(len[d] * sizeof(int));
-    o_ipos[d] = take(len[d] * sizeof(int));
-    if (p->gen[d]) o_gidx[d] = take(gidx[d].size() * sizeof(int));
+    o_rev[d] = take(rev[d].size() * sizeof(int));
+    o_ipos[d] = take(rev[d].size() * sizeof(int));
+    if (!gidx[d].empty()) o_gidx[d] = take(gidx[d].size() * sizeof(int));
   }
   const size_t int_bytes = off - o_int;
   const size_t o_status = take(sizeof(int));
@@ -922,52 +896,50 @@ int ff_plan_create(const int n[3], const double lo[3], const double hi[3], int p
     for (int d = 0; d < 3; d++) {
       int *hrev = reinterpret_cast<int *>(host.data() + (o_rev[d] - o_int));
       int *hpos = reinterpret_cast<int *>(host.data() + (o_ipos[d] - o_int));
-      for (int q = 0; q < len[d]; q++) {
+      for (int q = 0; q < (int)rev[d].size(); q++) {
         hrev[q] = rev[d][q];
         hpos[rev[d][q]] = q;
       }
-      if (p->gen[d]) std::memcpy(host.data() + (o_gidx[d] - o_int), gidx[d].data(), gidx[d].size() * sizeof(int));
+      if (!gidx[d].empty()) std::memcpy(host.data() + (o_gidx[d] - o_int), gidx[d].data(), gidx[d].size() * sizeof(int));
     }
     if (rc == FF_OK && cudaMemcpy(base + o_int, host.data(), int_bytes, cudaMemcpyHostToDevice) != cudaSuccess)
       rc = set_error(FF_ERR_CUDA, "ff_plan_create: table upload failed");
   }
   for (int d = 0; d < 3 && rc == FF_OK; d++) {
     const int L = len[d];
-    const int blocks = std::min(1024, (L + 255) / 256);
-    k_twiddles<<<blocks, 256>>>(L, reinterpret_cast<double2 *>(base + o_tw64[d]));
-    if (precision == FF_FP32) k_twiddles<<<blocks, 256>>>(L, reinterpret_cast<float2 *>(base + o_tw[d]));
-    const int cnt = d == 2 ? p->nh : n[d];
-    k_wavenumbers<<<std::min(1024, (cnt + 255) / 256), 256>>>(n[d], cnt, d != 2, p->dd[d],
-                                                              reinterpret_cast<double *>(base + o_kk[d]));
-    p->kk[d] = reinterpret_cast<double *>(base + o_kk[d]);
-    AxisDev<double2> ad{};
-    AxisDev<float2> af{};
-    ad.n = af.n = L;
-    ad.nstages = af.nstages = (int)radix[d].size();
-    for (size_t s = 0; s < radix[d].size(); s++) ad.radix[s] = af.radix[s] = radix[d][s];
-    ad.tw = reinterpret_cast<const double2 *>(base + o_tw[d]);
-    af.tw = reinterpret_cast<const float2 *>(base + o_tw[d]);
-    ad.tw64 = af.tw64 = reinterpret_cast<const double2 *>(base + o_tw64[d]);
-    ad.rev = af.rev = reinterpret_cast<const int *>(base + o_rev[d]);
-    ad.ipos = af.ipos = reinterpret_cast<const int *>(base + o_ipos[d]);
-    p->axd[d] = ad;
-    p->axf[d] = af;
+    if (!p->bsM[d]) {
+      const int blocks = std::min(1024, (L + 255) / 256);
+      k_twiddles<<<blocks, 256>>>(L, reinterpret_cast<double2 *>(base + o_tw64[d]));
+      if (precision == FF_FP32) k_twiddles<<<blocks, 256>>>(L, reinterpret_cast<float2 *>(base + o_tw[d]));
+      AxisDev<double2> ad{};
+      AxisDev<float2> af{};
+      ad.n = af.n = L;
+      ad.nstages = af.nstages = (int)radix[d].size();
+      for (size_t s = 0; s < radix[d].size(); s++) ad.radix[s] = af.radix[s] = radix[d][s];
+      ad.tw = reinterpret_cast<const double2 *>(base + o_tw[d]);
+      af.tw = reinterpret_cast<const float2 *>(base + o_tw[d]);
+      ad.tw64 = af.tw64 = reinterpret_cast<const double2 *>(base + o_tw64[d]);
+      ad.rev = af.rev = reinterpret_cast<const int *>(base + o_rev[d]);
+      ad.ipos = af.ipos = reinterpret_cast<const int *>(base + o_ipos[d]);
+      p->axd[d] = ad;
+      p->axf[d] = af;
+    }
+    const int *idx = reinterpret_cast<const int *>(base + o_gidx[d]);
     if (p->gen[d] && rc == FF_OK) {
-      const int *idx = reinterpret_cast<const int *>(base + o_gidx[d]);
-      rc = precision == FF_FP64 ? gen_axis_build(n[d], gradix[d], base + o_gen[d], idx, &p->gpd[d].ax)
-                                : gen_axis_build(n[d], gradix[d], base + o_gen[d], idx, &p->gpf[d].ax);
+      rc = precision == FF_FP64 ? gen_axis_build(L, gradix[d], base + o_gen[d], idx, &p->gpd[d].ax)
+                                : gen_axis_build(L, gradix[d], base + o_gen[d], idx, &p->gpf[d].ax);
     }
     if (p->bsM[d] && rc == FF_OK) {
-      const int *drev = reinterpret_cast<const int *>(base + o_rev[d]);
-      if (precision == FF_FP64) {
-        double2 *ch = reinterpret_cast<double2 *>(base + o_chirp[d]), *gh = reinterpret_cast<double2 *>(base + o_ghat[d]);
-        rc = bs_tables<double2>(n[d], L, drev, ch, gh);
-        p->bsd[d] = BsAxis<double2>{ad, n[d], ch, gh};
-      } else {
-        float2 *ch = reinterpret_cast<float2 *>(base + o_chirp[d]), *gh = reinterpret_cast<float2 *>(base + o_ghat[d]);
-        rc = bs_tables<float2>(n[d], L, drev, ch, gh);
-        p->bsf[d] = BsAxis<float2>{af, n[d], ch, gh};
-      }
+      auto build = [&](auto &bs) {
+        using BC = std::remove_const_t<std::remove_pointer_t<decltype(bs.chirp)>>;
+        BC *ch = reinterpret_cast<BC *>(base + o_chirp[d]), *gh = reinterpret_cast<BC *>(base + o_ghat[d]);
+        bs.n = n[d];
+        bs.chirp = ch;
+        bs.ghat = gh;
+        const int r = gen_axis_build(L, gradix[d], base + o_gen[d], idx, &bs.ax);
+        return r == FF_OK ? bs_tables<BC>(n[d], L, idx, gradix[d].back(), ch, gh) : r;
+      };
+      rc = precision == FF_FP64 ? build(p->bspd[d]) : build(p->bspf[d]);
     }
   }
   if (rc == FF_OK && cudaGetLastError() != cudaSuccess) rc = set_error(FF_ERR_CUDA, "ff_plan_create: table kernels");

@@ -77,6 +77,21 @@ def test_long_lengths(torch_cuda, ff, axis, precision):
         check(torch_cuda, ff, n, precision)
 
 
+# Bluestein axes: the smallest, odd and even, just below and above a change of
+# the tile's row width, the largest of the declared range
+FACTORS = [11, 13, 17, 22, 26, 31, 33, 34, 37, 44, 55, 61, 66, 77, 88, 97, 101, 110, 121, 127, 130, 143, 169, 187, 211,
+           241, 251, 254, 257, 289, 290, 293, 296, 307, 331, 341, 374, 419, 499, 509, 601, 701, 883, 887, 901]
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_lengths_with_larger_prime_factors(torch_cuda, ff, axis, precision):
+    for q, m in enumerate(FACTORS):
+        a, b = [(6, 10), (5, 27), (9, 33), (4, 21)][q % 4]
+        n = {0: (m, a, b), 1: (a, m, b), 2: (a, b, m)}[axis]
+        check(torch_cuda, ff, n, precision)
+
+
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("n", [(100, 90, 81), (96, 75, 80), (147, 98, 105), (200, 180, 160)])
 def test_grids_of_several_waves(torch_cuda, ff, n, precision):
