@@ -108,7 +108,7 @@ class Plan:
 
 
 class Batch:
-    """Many independent grids solved together: five persistent launches (one
+    """Many independent grids solved together: five launches (one
     per pass) over the tiles of all grids, captured once in a CUDA graph.
 
     dims: list of (ni, nj, nk); lo/hi: per-grid bounds or None for the

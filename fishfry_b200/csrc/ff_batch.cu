@@ -1,5 +1,5 @@
 // The batched form: many independent grids of uneven sizes solved by five
-// persistent launches (one per pass) captured once in a CUDA graph, with
+// launches (one per pass) captured once in a CUDA graph, with
 // tile shapes picked by a measuring autotuner.  Each grid's solve is the
 // single-grid algorithm (ParisPencil.cpp:95-425 restated as five passes).
 //
@@ -48,10 +48,9 @@ struct ff_batch {
   size_t csz = 16;
   std::vector<BatchGridHost> grids;
   std::vector<size_t> bytes;
-  void *dmem = nullptr;          // axis tables, status, tickets, descriptors, work lists
+  void *dmem = nullptr;          // axis tables, status, descriptors, work lists
   size_t dmem_size = 0;
   int *status = nullptr;
-  int *tickets = nullptr;        // one per pass
   void *desc = nullptr;          // device grid descriptors
   size_t desc_size = 0;
   unsigned char *desc_host = nullptr;   // pinned image of the descriptors
@@ -60,7 +59,7 @@ struct ff_batch {
   int2 *entries[5] = {};
   int *starts[5] = {};
   int ntiles[5] = {};
-  int blocks[5] = {};
+  int ahead[5] = {};             // blocks resident at once
   size_t smem[5] = {};
   bool desc_dirty = true;
   // axis tables by (length, radix order); default orders live in dmem, other
@@ -101,10 +100,10 @@ int pass_prepare(int precision, int kind, size_t smem, int *per_sm) {
 }
 
 int pass_launch(const ff_batch *b, int kind, cudaStream_t st) {
-  const BatchWork wl{b->entries[kind], b->starts[kind], b->count, b->tickets + kind};
+  const BatchWork wl{b->entries[kind], b->starts[kind], b->count, b->ahead[kind]};
   return b->precision == FF_FP64
-             ? batch_pass_launch<double>(kind, b->desc, b->maps, wl, b->blocks[kind], b->smem[kind], st)
-             : batch_pass_launch<float>(kind, b->desc, b->maps, wl, b->blocks[kind], b->smem[kind], st);
+             ? batch_pass_launch<double>(kind, b->desc, b->maps, wl, b->ntiles[kind], b->smem[kind], st)
+             : batch_pass_launch<float>(kind, b->desc, b->maps, wl, b->ntiles[kind], b->smem[kind], st);
 }
 
 }  // namespace
@@ -119,12 +118,13 @@ int batch_tiles_of(const BatchGridHost &g, int kind) {
   }
   const long planes = kind == 2 ? g.n[1] : g.n[0];
   if (s.tma) return (int)(planes * ((g.nh + s.W - 1) / s.W));
-  const long ncols = planes * g.nh;
+  // FP32 columns go in pairs: rows count their padding column
+  const long ncols = planes * g.nhp;
   return (int)((ncols + s.W - 1) / s.W);
 }
 
 size_t batch_shape_smem(int precision, const BatchGridHost &g, int kind, const TileShape &s) {
-  return batch_tile_smem(kind, batch_axis_len(g, kind), g.n[2], g.nhp, s.W, precision == FF_FP64 ? 16 : 8);
+  return batch_tile_smem(kind, batch_axis_len(g, kind), g.n[2], g.nhp, s.W, s.ct, precision == FF_FP64 ? 16 : 8);
 }
 
 // z passes of a runtime length may move line blocks by bulk copies when the
@@ -164,7 +164,9 @@ TileShape batch_default_shape(int precision, const BatchGridHost &g, int kind) {
     const size_t csz = precision == FF_FP64 ? 16 : 8;
     const int align = csz == 16 ? 8 : 16;
     const size_t per_pair = 2 * (size_t)((g.n[2] + align - 1) / align * align) * csz;
-    int W = std::max(1, 1024 / std::max(1, g.n[2]));
+    // FP32 tiles of compile-time lengths: twice that (their lines are half as
+    // long in bytes; 60 grids of 32 to 128 points: z passes 110 / 110 -> 94 / 92 us)
+    int W = std::max(1, (precision == FF_FP32 && s.ct ? 2048 : 1024) / std::max(1, g.n[2]));
     W = std::max(W, (int)std::max<size_t>(1, std::min<size_t>(8, (32 * 1024) / per_pair)));
     W = (int)std::min<long>(W, npairs);
     while (W > 1 && !batch_shape_valid(precision, g, kind, TileShape{W, s.ct, 0})) W--;
@@ -363,7 +365,7 @@ int build_work(ff_batch *b) {
     int rc = pass_prepare(b->precision, k, smem, &per_sm);
     if (rc != FF_OK) return rc;
     if (per_sm < 1) return set_error(FF_ERR_UNSUPPORTED, "batch pass %d: a tile does not fit on an SM", k);
-    b->blocks[k] = std::max(1, std::min(b->ntiles[k], per_sm * b->num_sms));
+    b->ahead[k] = per_sm * b->num_sms;
     FF_CUDA(cudaMemcpy(b->entries[k], ent.data(), ent.size() * sizeof(int2), cudaMemcpyHostToDevice));
     FF_CUDA(cudaMemcpy(b->starts[k], start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice));
   }
@@ -378,11 +380,10 @@ void drop_graph(ff_batch *b) {
   b->graph = nullptr;
 }
 
-// The five passes (and a reset of the tickets, and the phase events), as
+// The five passes (and the phase events), as
 // issued on `st`; captured once into the graph.  The events are recorded as
 // external event nodes, so the host can wait on and time them after a replay.
 int issue_passes(ff_batch *b, cudaStream_t st) {
-  FF_CUDA(cudaMemsetAsync(b->tickets, 0, 5 * sizeof(int), st));
   FF_CUDA(cudaEventRecordWithFlags(b->ev[0], st, cudaEventRecordExternal));
   for (int k = 0; k < 5; k++) {
     int rc = pass_launch(b, k, st);
@@ -456,7 +457,6 @@ int take_status(ff_batch *b, cudaStream_t st) {
 int time_pass(ff_batch *b, int kind, cudaStream_t st, int reps, float *ms) {
   std::vector<float> t;
   for (int r = 0; r <= reps; r++) {
-    FF_CUDA(cudaMemsetAsync(b->tickets + kind, 0, sizeof(int), st));
     FF_CUDA(cudaEventRecord(b->ev[0], st));
     int rc = pass_launch(b, kind, st);
     if (rc != FF_OK) return rc;
@@ -497,7 +497,6 @@ int batch_create_core(ff_batch *b, int count, const int *dims, const double *lo,
       if (!table_of.count(n)) table_of[n] = take(batch_axis_bytes(n, precision));
     }
   const size_t o_status = take(sizeof(int));
-  const size_t o_tickets = take(5 * sizeof(int));
   const size_t o_desc = take((size_t)count * b->desc_size);
   const size_t o_maps = take((size_t)count * 2 * sizeof(CUtensorMap));
   size_t o_ent[5], o_start[5];
@@ -518,7 +517,6 @@ int batch_create_core(ff_batch *b, int count, const int *dims, const double *lo,
   }
   char *base = static_cast<char *>(b->dmem);
   b->status = reinterpret_cast<int *>(base + o_status);
-  b->tickets = reinterpret_cast<int *>(base + o_tickets);
   b->desc = base + o_desc;
   b->maps = reinterpret_cast<CUtensorMap *>(base + o_maps);
   for (int k = 0; k < 5; k++) {

@@ -4,8 +4,7 @@
 //
 // A batch runs the same five passes as a single solve (z R2C, y forward,
 // x forward + filter + inverse, y inverse, z C2R), but every launch covers
-// the tiles of all its grids: one persistent kernel per pass, whose blocks
-// take tiles from a ticket counter until the work list is exhausted.
+// the tiles of all its grids: one launch per pass, one block per tile.
 #pragma once
 
 #include <cuda.h>
@@ -17,6 +16,7 @@
 #include <vector>
 
 #include "ff_fft.cuh"
+#include "ff_gen.hpp"
 
 namespace ff {
 
@@ -45,14 +45,19 @@ inline bool batch_special_n(int n) {
   return false;
 }
 
+constexpr int kBatchPadRows = 7;
+// Stages of a runtime plan: lengths up to 574 in radices 8, 4, 2, 5, 3, 7 have at
+// most 6 (486 = 2 * 3^5).
+constexpr int kBatchStages = 6;
+
 // One launch: tiles of entries e = 0..nentry-1 are numbered start[e] ..
-// start[e+1]-1; entry e names (grid, pass).  ticket is zeroed before the
-// launch.
+// start[e+1]-1; entry e names (grid, pass).  ahead: tiles (blocks) resident at
+// once; the z passes hint the input of the tile that far on into L2.
 struct BatchWork {
   const int2 *entry;
   const int *start;
   int nentry;
-  int *ticket;
+  int ahead;
 };
 
 // Tile shape of one pass of one grid: z passes take W line pairs per tile;
@@ -81,8 +86,11 @@ constexpr int kBatchOrders = 3;
 std::vector<int> batch_radix_order(int n, int order);
 
 // Shared memory of one tile (bytes, with alignment slack).
-inline size_t batch_tile_smem(int kind, int n_axis, int nk, int nhp, int W, size_t csz) {
+inline size_t batch_tile_smem(int kind, int n_axis, int nk, int nhp, int W, int ct, size_t csz) {
   if (kind == 0 || kind == 4) {
+    // runtime plans: tiles of ff_gen_lines.cuh, with at most kBatchPadRows rows
+    // of padding (the first radix is at most 8)
+    if (!ct) return gen_line_smem(nk, nhp, (int)csz / 2, nk + kBatchPadRows, W);
     const int align = csz == 16 ? 8 : 16;
     const size_t P = (size_t)(nk + align - 1) / align * align;
     const size_t a = std::max<size_t>((size_t)W * P, 2 * (size_t)W * nhp) * csz;

@@ -42,7 +42,7 @@ __device__ __forceinline__ void bs_conv(const BsPass<C> &a, const GenLane &ln, V
   const int S = ax.S;   // n >= 11, so M >= 21: at least two stages
   const TileLoad<V> ld{tile, a.lu, ln.c};
   const TilePut<V> back{tile, a.lu, ln.c};
-  gen_dif<WAY, false>(ax, S - 1, ln, tile, a.lu, ld0);
+  gen_dif<WAY, false>(ax.st, S - 1, PackedTw<C>{ax.tw}, ln, tile, a.lu, ld0);
   with_gen_radix(ax.st[S - 1].R, [&](auto tag) {
     // the last DIF stage, the product with ghat and the first DIT stage on one
     // register group (the span-R stages have no twiddles)
@@ -62,8 +62,8 @@ __device__ __forceinline__ void bs_conv(const BsPass<C> &a, const GenLane &ln, V
   for (int s = S - 2; s >= 0; s--) {
     with_gen_radix(ax.st[s].R, [&](auto tag) {
       constexpr int R = decltype(tag)::value;
-      if (s > 0) gen_stage<WAY, R, true, true, V>(ax.st[s], ax.tw, ln, ld, back);
-      else gen_stage<WAY, R, true, true, V>(ax.st[0], ax.tw, ln, ld, put);
+      if (s > 0) gen_stage<WAY, R, true, true, V>(ax.st[s], PackedTw<C>{ax.tw}, ln, ld, back);
+      else gen_stage<WAY, R, true, true, V>(ax.st[0], PackedTw<C>{ax.tw}, ln, ld, put);
     });
     __syncthreads();
   }
@@ -378,7 +378,7 @@ GenShape bs_shape(int kind, int ni, int nj, int nk, int nhp, int esz, int M, int
   const int cu = 16 / (2 * esz);
   if (kind == 0 || kind == 4) {
     s.tile_rows = M;
-    gen_z_shape(&s, ni, nj, nk, nhp, esz, num_sms);
+    gen_z_shape(&s, ni, nj, nk, nhp, esz, num_sms, false);
     return s;
   }
   const int nh = nk / 2 + 1;

@@ -29,7 +29,7 @@
 
 namespace ff {
 
-constexpr int kMaxStages = 16;
+constexpr int kMaxStages = 8;   // radices 8, 4, 2, 5, 3, 7: at most 7 stages up to 4096 points (3^7, 2 * 3^6)
 
 template <typename T> struct Cplx;
 template <> struct Cplx<double> { using type = double2; };
@@ -856,14 +856,17 @@ __device__ __forceinline__ void l2_prefetch(const void *src, uint32_t bytes) {
 }
 
 // Element copies from global to shared memory that complete asynchronously
-// (all of a thread's copies are in flight together); 16 bytes (.cg, L2 only)
-// or 8 bytes (.ca); addresses aligned to the size.  cp_async_wait_all waits
+// (all of a thread's copies are in flight together); 16 bytes (.cg, L2 only),
+// 8 or 4 bytes (.ca); addresses aligned to the size.  cp_async_wait_all waits
 // for this thread's copies; a barrier then publishes them to the block.
 __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async8(void *dst, const void *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void *dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");

@@ -120,6 +120,30 @@ void gen_stages(int n, const std::vector<int> &radix, int pad, int threads, int 
   }
 }
 
+void gen_line_stages(int n, const std::vector<int> &radix, int pad, int threads, bool table, int *S, GenStage *st) {
+  gen_stages(n, radix, pad, 1, 1, S, st);
+  int step = 1;
+  for (int s = 0; s < *S; s++) {
+    if (table) st[s].tw = step;
+    step *= st[s].R;
+  }
+  st[*S] = GenStage{};
+  st[*S].nb = st[*S - 1].nb / 2 + 1;   // frequency bases 0 .. nR/2
+  for (int s = 0; s <= *S; s++) {
+    st[s].inv_nb = 1.0f / (float)st[s].nb;
+    st[s].dq = threads / st[s].nb;
+    st[s].dr = threads % st[s].nb;
+  }
+}
+
+size_t gen_line_smem(int nk, int nhp, int esz, int tile_rows, int W) {
+  const int cu = 16 / (2 * esz), units = (W + cu - 1) / cu;
+  const size_t lines = (size_t)2 * cu * units;
+  const size_t tile = ((size_t)tile_rows * (units | 1) * 16 + 127) & ~size_t(127);
+  const size_t stage = std::max(lines * nk * esz + 16, lines * nhp * 2 * esz);
+  return tile + ((stage + 127) & ~size_t(127)) + 128;
+}
+
 namespace {
 
 size_t r256(size_t b) { return (b + 255) & ~size_t(255); }
@@ -198,7 +222,7 @@ void gen_pick_threads(GenShape *s) {
   s->threads = std::min(256, std::max(64, 768 / blocks / 32 * 32));
 }
 
-void gen_z_shape(GenShape *s, int ni, int nj, int nk, int nhp, int esz, int num_sms) {
+void gen_z_shape(GenShape *s, int ni, int nj, int nk, int nhp, int esz, int num_sms, bool lines_kind) {
   const int cu = 16 / (2 * esz);   // line pairs per unit
   const long nlines = (long)ni * nj;
   // many small tiles (up to 40 KB, five or more blocks on an SM) beat fewer
@@ -218,6 +242,7 @@ void gen_z_shape(GenShape *s, int ni, int nj, int nk, int nhp, int esz, int num_
     const size_t stage = std::max((size_t)lines * s->lp * esz + 16, (size_t)lines * s->sp * 2 * esz);
     s->smem = tile + ((stage + 127) & ~size_t(127)) + 128;
     s->grid = (nlines + lines - 1) / lines;
+    if (lines_kind) s->smem = gen_line_smem(nk, nhp, esz, s->tile_rows, s->units * cu);
     if (s->units == 1) break;
     if (s->smem <= limit && (s->grid >= num_sms || s->units <= 2)) break;
   }
@@ -229,7 +254,7 @@ GenShape gen_shape(int kind, int ni, int nj, int nk, int nhp, int esz, const std
   const int cu = 16 / (2 * esz);   // complex columns (or line pairs) per unit
   if (kind == 0 || kind == 4) {
     s.tile_rows = nk + gen_pad(nk, radix) * (radix[0] - 1);
-    gen_z_shape(&s, ni, nj, nk, nhp, esz, num_sms);
+    gen_z_shape(&s, ni, nj, nk, nhp, esz, num_sms, esz == 4);
     return s;
   }
   const int n = kind == 2 ? ni : nj;

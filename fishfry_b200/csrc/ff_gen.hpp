@@ -25,6 +25,7 @@ struct GenStage {
   int nb;       // butterflies per column, n / R
   int dq, dr;   // step / m, step % m
   float inv_m;  // 1 / m, correctly rounded
+  float inv_nb; // tiles with butterflies fastest (gen_line_stages): 1 / nb
   int ms;       // rows of the tile between a butterfly's points
   float inv_pb; // z passes: 1 / blocks of this stage in a block of stage 0 (0: rows are not padded)
   int tw;       // offset of the stage's twiddles in the table (complex values)
@@ -34,7 +35,7 @@ struct GenStage {
 // [j][r], r < Rp = R rounded up to even: entry (j, r) = exp(-2 pi i j r / L).
 template <typename C> struct GenAxis {
   int n, S;
-  GenStage st[kGenMaxStages];
+  GenStage st[kGenMaxStages + 1];   // gen_line_stages: st[S] counts the split's items
   const C *tw;        // per-stage twiddles, in C's precision (FP64-generated)
   // strided passes: last-stage group g -> frequency base k0 (the group's R
   // frequencies are k0 + r n/R); z passes: k0 -> first tile row of its group
@@ -61,6 +62,14 @@ std::vector<int> gen_bases(int n, const std::vector<int> &radix);
 int gen_table_size(int n, const std::vector<int> &radix);
 void gen_stages(int n, const std::vector<int> &radix, int pad, int threads, int units, int *S, GenStage *st);
 
+// The same for z tiles with butterflies fastest (ff_gen_lines.cuh): a thread
+// takes items t, t + threads, ... of all columns and keeps (column, butterfly) by
+// adding (dq, dr) = (threads / nb, threads % nb); st[S] counts the items of the
+// forward split.  table: the twiddle steps of an axis's plain table instead of
+// packed offsets.  Shared memory of such a tile of W line pairs.
+void gen_line_stages(int n, const std::vector<int> &radix, int pad, int threads, bool table, int *S, GenStage *st);
+size_t gen_line_smem(int nk, int nhp, int esz, int tile_rows, int W);
+
 // A tile is `units` columns of 16 bytes (one FP64 or two adjacent FP32 complex
 // values; z passes: one FP64 line pair or two FP32 ones) by n rows.
 struct GenShape {
@@ -78,9 +87,9 @@ struct GenShape {
 GenShape gen_shape(int kind, int ni, int nj, int nk, int nhp, int esz, const std::vector<int> &radix, int num_sms);
 
 // Parts of gen_shape that other tiles share: units, pitches, shared memory and
-// grid of a z pass whose tile has s->tile_rows rows; threads per block from the
-// shared memory.
-void gen_z_shape(GenShape *s, int ni, int nj, int nk, int nhp, int esz, int num_sms);
+// grid of a z pass whose tile has s->tile_rows rows (lines_kind: a tile with
+// butterflies fastest); threads per block from the shared memory.
+void gen_z_shape(GenShape *s, int ni, int nj, int nk, int nhp, int esz, int num_sms, bool lines_kind);
 void gen_pick_threads(GenShape *s);
 
 // Cost of an n-point transform's stages per point (arbitrary unit).

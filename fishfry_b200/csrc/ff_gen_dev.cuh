@@ -31,7 +31,7 @@
 // z 245 -> 350 us).  64 registers and 32 warps spill (y 217 -> 247 us).
 #pragma once
 
-#include "ff_gen_stages.cuh"
+#include "ff_gen_lines.cuh"
 
 namespace ff {
 
@@ -72,7 +72,7 @@ __device__ __forceinline__ void gen_x_tile(const GenPass<C> &a, const GenLane &l
   const int S = a.ax.S;
   const TileLoad<V> ld{tile, a.lu, ln.c};
   const TilePut<V> put{tile, a.lu, ln.c};
-  gen_dif<GenStrided<C>, false>(a.ax, S - 1, ln, tile, a.lu, ld);
+  gen_dif<GenStrided<C>, false>(a.ax.st, S - 1, PackedTw<C>{a.ax.tw}, ln, tile, a.lu, ld);
   {
     constexpr int CU = 16 / sizeof(C);
     const GenStage &s = a.ax.st[S - 1];
@@ -100,7 +100,7 @@ __device__ __forceinline__ void gen_x_tile(const GenPass<C> &a, const GenLane &l
   }
   for (int s = S - 2; s >= 0; s--) {
     with_gen_radix(a.ax.st[s].R, [&](auto tag) {
-      gen_stage<GenStrided<C>, decltype(tag)::value, true, true, V>(a.ax.st[s], a.ax.tw, ln, ld, put);
+      gen_stage<GenStrided<C>, decltype(tag)::value, true, true, V>(a.ax.st[s], PackedTw<C>{a.ax.tw}, ln, ld, put);
     });
     __syncthreads();
   }
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(256, 3)
     }
   } else {
     const TileLoad<V> ld{tile, a.lu, ln.c};
-    gen_dif<GenStrided<C>, KIND == 3>(a.ax, a.ax.S - 1, ln, tile, a.lu, ld);
+    gen_dif<GenStrided<C>, KIND == 3>(a.ax.st, a.ax.S - 1, PackedTw<C>{a.ax.tw}, ln, tile, a.lu, ld);
     gen_y_last<KIND == 3>(a, ln, tile, dst + (long)o * a.nj * a.nhp, kt * W);
   }
 }
@@ -165,6 +165,47 @@ __global__ void __launch_bounds__(256, 3)
 // staging area (real lines of pitch lp on one side, spectrum rows of pitch sp
 // on the other).  Lines at or past the end are zero in and not stored.
 //
+// FP32: z tiles with butterflies fastest (ff_gen_lines.cuh), whose unpadded
+// staging moves by one copy each way: 480x400x360 z 162 / 160 -> 141 / 143 us,
+// 640x640x320 306 / 296 -> 242 / 254.  (FP64 lost with them: 243 / 240 -> 250 /
+// 260 and 480^3 368 / 349 -> 410 / 429, their last rows and twiddles being twice
+// as wide; it keeps units fastest.)
+template <int KIND>
+__global__ void __launch_bounds__(256, 3)
+    k_gen_lines(const void *in, void *out, const __grid_constant__ GenPass<float2> a) {
+  extern __shared__ unsigned char smraw[];
+  __shared__ __align__(8) uint64_t mbar;
+  const long nlines = (long)a.ni * a.nj;
+  const LineTileOf<float2> b =
+      line_tile<float2>(a.nk, a.nhp, nlines, 2 << a.lu, a.tile_rows, blockIdx.x, align128(smraw));
+  // rows in and out, in bytes
+  const size_t rin = KIND == 0 ? a.nk * sizeof(float) : a.nhp * sizeof(float2);
+  const unsigned char *src = static_cast<const unsigned char *>(in);
+  if (threadIdx.x == 0) {
+    mbar_init(&mbar, 1);
+    mbar_init_fence();
+    // one copy rounded up to 16 bytes: a real field's buffer also holds the
+    // half spectrum, which is longer; spectrum rows are 16-byte multiples
+    const uint32_t bytes = (uint32_t)(b.nl * rin + 15) & ~15u;
+    mbar_expect_tx(&mbar, bytes);
+    bulk_load(b.raw, src + b.line0 * rin, bytes, &mbar);
+  }
+  if (threadIdx.x == blockDim.x - 1 && a.l2_ahead > 0) {
+    const long fl = b.line0 + (long)a.l2_ahead * b.lines;
+    if (fl < nlines) l2_prefetch(src + fl * rin, (uint32_t)(min((long)b.lines, nlines - fl) * rin) & ~15u);
+  }
+  __syncthreads();
+  if (!z_wait(&mbar, a.status, a.wait_iters)) return;
+  const PackedTw<float2> tw{a.ax.tw};
+  auto row_of = [&](int k0) { return __ldg(a.ax.idx + k0); };
+  if constexpr (KIND == 0) line_forward(b, a.ax.st, a.ax.S, tw, row_of);
+  else line_inverse(b, a.ax.st, a.ax.S, tw, row_of);
+  fence_proxy_async_smem();
+  __syncthreads();
+  if constexpr (KIND == 0) bulk_out(static_cast<float2 *>(out) + b.line0 * a.nhp, b.rows, (size_t)b.nl * a.nhp);
+  else bulk_out(static_cast<float *>(out) + b.line0 * a.nk, b.raw, (size_t)b.nl * a.nk);
+}
+
 // R2C of the real lines (ParisPencil.cpp:152-165).
 template <typename T>
 __global__ void __launch_bounds__(256, 3)
@@ -214,7 +255,7 @@ __global__ void __launch_bounds__(256, 3)
   };
   const int S = a.ax.S;
   if (S > 1) {
-    gen_dif<GenLines, false>(a.ax, S - 1, ln, tile, a.lu, ld0);
+    gen_dif<GenLines, false>(a.ax.st, S - 1, PackedTw<C>{a.ax.tw}, ln, tile, a.lu, ld0);
   } else {
     // one stage: the split reads the tile
     for (int pos = ln.b0; pos < nk; pos += ln.step) ld0(pos, pos, a.ax.st[0], tile + (pos << a.lu) + ln.c, RadixTag<1>{});
@@ -309,7 +350,7 @@ __global__ void __launch_bounds__(256, 3)
   };
   const int S = a.ax.S;
   if (S > 1) {
-    gen_dif<GenLines, true>(a.ax, S - 1, ln, tile, a.lu, ld0);
+    gen_dif<GenLines, true>(a.ax.st, S - 1, PackedTw<C>{a.ax.tw}, ln, tile, a.lu, ld0);
   } else {
     for (int pos = ln.b0; pos < nk; pos += ln.step) ld0(pos, pos, a.ax.st[0], tile + (pos << a.lu) + ln.c, RadixTag<1>{});
     __syncthreads();
@@ -353,11 +394,15 @@ __global__ void __launch_bounds__(256, 3)
 // ----------------------------------------------------------------- launches
 template <typename T> const void *gen_kernel(int kind) {
   switch (kind) {
-    case 0: return (const void *)k_gen_zfwd<T>;
+    case 0:
+      if constexpr (sizeof(T) == 4) return (const void *)k_gen_lines<0>;
+      else return (const void *)k_gen_zfwd<T>;
     case 1: return (const void *)k_gen_strided<T, 1>;
     case 2: return (const void *)k_gen_strided<T, 2>;
     case 3: return (const void *)k_gen_strided<T, 3>;
-    default: return (const void *)k_gen_zinv<T>;
+    default:
+      if constexpr (sizeof(T) == 4) return (const void *)k_gen_lines<4>;
+      else return (const void *)k_gen_zinv<T>;
   }
 }
 
@@ -377,11 +422,17 @@ int gen_launch(int kind, const GenPass<typename Cplx<T>::type> &a, const GenShap
   using C = typename Cplx<T>::type;
   const unsigned grid = (unsigned)s.grid;
   switch (kind) {
-    case 0: k_gen_zfwd<T><<<grid, s.threads, s.smem, st>>>(static_cast<const T *>(in), static_cast<C *>(out), a); break;
+    case 0:
+      if constexpr (sizeof(T) == 4) k_gen_lines<0><<<grid, s.threads, s.smem, st>>>(in, out, a);
+      else k_gen_zfwd<T><<<grid, s.threads, s.smem, st>>>(static_cast<const T *>(in), static_cast<C *>(out), a);
+      break;
     case 1: k_gen_strided<T, 1><<<grid, s.threads, s.smem, st>>>(*map, static_cast<C *>(out), a); break;
     case 2: k_gen_strided<T, 2><<<grid, s.threads, s.smem, st>>>(*map, static_cast<C *>(out), a); break;
     case 3: k_gen_strided<T, 3><<<grid, s.threads, s.smem, st>>>(*map, static_cast<C *>(out), a); break;
-    default: k_gen_zinv<T><<<grid, s.threads, s.smem, st>>>(static_cast<const C *>(in), static_cast<T *>(out), a); break;
+    default:
+      if constexpr (sizeof(T) == 4) k_gen_lines<4><<<grid, s.threads, s.smem, st>>>(in, out, a);
+      else k_gen_zinv<T><<<grid, s.threads, s.smem, st>>>(static_cast<const C *>(in), static_cast<T *>(out), a);
+      break;
   }
   FF_CUDA(cudaGetLastError());
   return FF_OK;

@@ -228,9 +228,8 @@ template <bool INV, typename V> struct UDft<9, INV, V> {
 // FP64 loads w (radices from 6 also w^h, h = R/2 rounded up, which halves the
 // chain of products and its rounding) and forms the other powers (loading every
 // factor measured slower), FP32 loads them two at a time.
-template <int R, bool CONJ>
-__device__ __forceinline__ void gen_twiddle(double2 *v, const double2 *__restrict__ t) {
-  const double2 w1 = __ldg(t + 1);
+template <int R, bool CONJ, typename WH>
+__device__ __forceinline__ void gen_powers(double2 *v, double2 w1, WH &&half) {
   double2 w = w1;
   if constexpr (R < 6) {
 #pragma unroll
@@ -240,7 +239,7 @@ __device__ __forceinline__ void gen_twiddle(double2 *v, const double2 *__restric
     }
   } else {
     constexpr int H = (R + 1) / 2;
-    const double2 wh = __ldg(t + H);
+    const double2 wh = half();
     v[H] = ucmul<CONJ>(v[H], wh);
 #pragma unroll
     for (int r = 1; r < H; r++) {
@@ -249,6 +248,10 @@ __device__ __forceinline__ void gen_twiddle(double2 *v, const double2 *__restric
       if (r + 1 < H) w = cmul(w, w1);
     }
   }
+}
+template <int R, bool CONJ>
+__device__ __forceinline__ void gen_twiddle(double2 *v, const double2 *__restrict__ t) {
+  gen_powers<R, CONJ>(v, __ldg(t + 1), [&] { return __ldg(t + (R + 1) / 2); });
 }
 template <int R, bool CONJ> __device__ __forceinline__ void gen_twiddle(FPair *v, const float2 *__restrict__ t) {
   const float4 *t4 = reinterpret_cast<const float4 *>(t);
@@ -259,6 +262,29 @@ template <int R, bool CONJ> __device__ __forceinline__ void gen_twiddle(FPair *v
     if (r + 1 < R) v[r + 1] = ucmul<CONJ>(v[r + 1], make_float2(w.z, w.w));
   }
 }
+
+// Twiddles of the packed per-stage tables (GenAxis) and of an axis's plain table
+// (AxisDev: entry q = exp(-2 pi i q / n); GenStage::tw is then the step n / L).
+template <typename C> struct PackedTw {
+  const C *tw;
+  template <int R, bool CONJ, typename V> __device__ __forceinline__ void apply(V *v, const GenStage &s, int j) const {
+    gen_twiddle<R, CONJ>(v, tw + s.tw + j * ((R + 1) & ~1));
+  }
+};
+template <typename C> struct AxisTw;
+template <> struct AxisTw<double2> {
+  const double2 *tw;
+  template <int R, bool CONJ> __device__ __forceinline__ void apply(double2 *v, const GenStage &s, int j) const {
+    gen_powers<R, CONJ>(v, __ldg(tw + j * s.tw), [&] { return __ldg(tw + j * ((R + 1) / 2) * s.tw); });
+  }
+};
+template <> struct AxisTw<float2> {
+  const float2 *tw;
+  template <int R, bool CONJ> __device__ __forceinline__ void apply(FPair *v, const GenStage &s, int j) const {
+#pragma unroll
+    for (int r = 1; r < R; r++) v[r] = ucmul<CONJ>(v[r], __ldg(tw + j * r * s.tw));
+  }
+};
 
 // The thread's place in a tile.
 struct GenLane {
@@ -307,10 +333,8 @@ template <typename V> struct TilePut {
 // A stage: ld(row, pos, s, v) fills a butterfly's R points (positions pos + r m,
 // tile rows row + r ms), put(row, pos, s, v) takes the result.  The thread walks
 // its butterflies b0, b0 + step, ... of the column.
-template <typename WAY, int R, bool INV, bool DIT, typename V, typename C, typename LD, typename ST>
-__device__ __forceinline__ void gen_stage(const GenStage &s, const C *__restrict__ tw, const GenLane &ln, LD &&ld,
-                                          ST &&put) {
-  constexpr int RP = (R + 1) & ~1;
+template <typename WAY, int R, bool INV, bool DIT, typename V, typename TW, typename LD, typename ST>
+__device__ __forceinline__ void gen_stage(const GenStage &s, const TW &tw, const GenLane &ln, LD &&ld, ST &&put) {
   constexpr RadixTag<R> tag{};
   // tile to tile: one pointer and stride for both sides
   constexpr bool kPut = std::is_same<std::decay_t<ST>, TilePut<V>>::value;
@@ -349,10 +373,9 @@ __device__ __forceinline__ void gen_stage(const GenStage &s, const C *__restrict
   // rows of the blocks of stage 0 are padded apart: one row each
   auto row_of = [&](int pos) { return WAY::kPad ? pos + __float2int_rz(((float)q + 0.5f) * s.inv_pb) : pos; };
   auto work = [&](V *v, int jj) {
-    const C *t = tw + s.tw + jj * RP;
-    if (DIT && s.m > 1) gen_twiddle<R, INV>(v, t);
+    if (DIT && s.m > 1) tw.template apply<R, INV>(v, s, jj);
     UDft<R, INV, V>::run(v);
-    if (!DIT && s.m > 1) gen_twiddle<R, INV>(v, t);
+    if (!DIT && s.m > 1) tw.template apply<R, INV>(v, s, jj);
   };
   int b = ln.b0;
   if constexpr (R <= WAY::kPair) {
@@ -411,18 +434,19 @@ template <typename F> __device__ __forceinline__ void with_split_radix(int r, F 
 
 // DIF stages 0 .. s1-1 in the tile, each followed by a barrier; the first reads
 // through ld0.
-template <typename WAY, bool INV, typename V, typename C, typename LD0>
-__device__ __forceinline__ void gen_dif(const GenAxis<C> &ax, int s1, const GenLane &ln, V *tile, int lu, LD0 &&ld0) {
+template <typename WAY, bool INV, typename V, typename TW, typename LD0>
+__device__ __forceinline__ void gen_dif(const GenStage *st, int s1, const TW &tw, const GenLane &ln, V *tile, int lu,
+                                        LD0 &&ld0) {
   const TileLoad<V> ld{tile, lu, ln.c};
   const TilePut<V> put{tile, lu, ln.c};
   for (int s = 0; s < s1; s++) {
-    with_gen_radix(ax.st[s].R, [&](auto tag) {
+    with_gen_radix(st[s].R, [&](auto tag) {
       constexpr int R = decltype(tag)::value;
       if constexpr (std::is_same<std::decay_t<LD0>, TileLoad<V>>::value) {
-        gen_stage<WAY, R, INV, false, V>(ax.st[s], ax.tw, ln, ld, put);
+        gen_stage<WAY, R, INV, false, V>(st[s], tw, ln, ld, put);
       } else {
-        if (s == 0) gen_stage<WAY, R, INV, false, V>(ax.st[s], ax.tw, ln, ld0, put);
-        else gen_stage<WAY, R, INV, false, V>(ax.st[s], ax.tw, ln, ld, put);
+        if (s == 0) gen_stage<WAY, R, INV, false, V>(st[s], tw, ln, ld0, put);
+        else gen_stage<WAY, R, INV, false, V>(st[s], tw, ln, ld, put);
       }
     });
     __syncthreads();

@@ -83,7 +83,6 @@ template <typename T> PassArgs<T> pass_args(const ff_plan *p) {
   for (int d = 0; d < 3; d++) {
     if constexpr (sizeof(T) == 8) a.ax[d] = p->axd[d];
     else a.ax[d] = p->axf[d];
-    a.kk[d] = nullptr;
   }
   a.invN = 1.0 / (double(p->n[0]) * double(p->n[1]) * double(p->n[2]));
   for (int d = 0; d < 3; d++) a.dd[d] = p->dd[d];

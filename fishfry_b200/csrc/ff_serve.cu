@@ -5,7 +5,7 @@
 // HBM budget (one arena, allocated at creation, sub-allocated best-fit) and a
 // cap on descriptor slots; an admitted request's field is copied into its
 // arena buffer, and from then on every scheduling step carries it one pass
-// further.  A step is, per precision, one persistent launch per pass kind
+// further.  A step is, per precision, one launch per pass kind
 // present (the batch kernels of ff_batch_dev.cuh) over the tiles of every
 // request at that pass, so requests that arrive while others run join the
 // next step and their work shares the launches.  Axis tables (twiddles,
@@ -127,7 +127,7 @@ struct Lane {
   CUtensorMap *maps = nullptr;             // device tensor maps [slots][2] (y, x boxes of the potential)
   CUtensorMap *maps_host = nullptr;        // pinned image
   std::vector<int> free_slots;
-  // ring buffers: per step r and kind k: entries [slots] int2, starts [slots + 1] int, 5 tickets
+  // ring buffers: per step r and kind k: entries [slots] int2, starts [slots + 1] int
   void *ring_dev = nullptr;
   unsigned char *ring_host = nullptr;
   size_t ring_bytes = 0;                   // one step's block
@@ -185,7 +185,7 @@ namespace {
 
 size_t step_block_bytes(int slots) {
   auto r = [](size_t b) { return (b + 255) & ~size_t(255); };
-  return 5 * (r(slots * sizeof(int2)) + r((slots + 1) * sizeof(int))) + r(5 * sizeof(int));
+  return 5 * (r(slots * sizeof(int2)) + r((slots + 1) * sizeof(int)));
 }
 
 int lane_init(ff_server *s, Lane &L, int precision) {
@@ -336,7 +336,7 @@ int issue_step(ff_server *s, Lane &L, bool *issued) {
   }
   if (members.empty()) return FF_OK;
   // compact layout of this step's work lists in ring block r: per kind the
-  // entries (int2) and the prefix sums (int), then the five tickets
+  // entries (int2) and the prefix sums (int)
   int cnt[5] = {0, 0, 0, 0, 0};
   for (uint64_t id : members) cnt[s->reqs[id].next_pass]++;
   size_t e_off[5], s_off[5], off = 0;
@@ -346,11 +346,10 @@ int issue_step(ff_server *s, Lane &L, bool *issued) {
     s_off[k] = off;
     off += ((cnt[k] + 1) * sizeof(int) + 7) & ~size_t(7);
   }
-  const size_t t_off = off;
-  off += 5 * sizeof(int);
   unsigned char *hb = L.ring_host + (size_t)r * L.ring_bytes;
   char *db = static_cast<char *>(L.ring_dev) + (size_t)r * L.ring_bytes;
   int fill[5] = {0, 0, 0, 0, 0};
+  size_t smem[5] = {0, 0, 0, 0, 0};
   for (int k = 0; k < 5; k++) reinterpret_cast<int *>(hb + s_off[k])[0] = 0;
   for (uint64_t id : members) {
     Request &q = s->reqs[id];
@@ -371,23 +370,22 @@ int issue_step(ff_server *s, Lane &L, bool *issued) {
     int *st = reinterpret_cast<int *>(hb + s_off[k]);
     reinterpret_cast<int2 *>(hb + e_off[k])[fill[k]] = make_int2(q.slot, k);
     st[fill[k] + 1] = st[fill[k]] + batch_tiles_of(q.g, k);
+    smem[k] = std::max(smem[k], batch_shape_smem(q.precision, q.g, k, q.g.shape[k]));
     fill[k]++;
     q.next_pass++;
     if (q.next_pass == 5) q.finish_step = L.next_step;
   }
-  std::memset(hb + t_off, 0, 5 * sizeof(int));
   FF_CUDA(cudaMemcpyAsync(db, hb, off, cudaMemcpyHostToDevice, L.stream));
   FF_CUDA(cudaEventRecord(L.fork_ev, L.stream));
   for (int k = 0; k < 5; k++) {
     if (!cnt[k]) continue;
     const BatchWork wl{reinterpret_cast<const int2 *>(db + e_off[k]), reinterpret_cast<const int *>(db + s_off[k]),
-                       cnt[k], reinterpret_cast<int *>(db + t_off) + k};
+                       cnt[k], batch_blocks_per_sm(k) * s->num_sms};
     const int tiles = reinterpret_cast<int *>(hb + s_off[k])[cnt[k]];
-    const int blocks = std::max(1, std::min(tiles, batch_blocks_per_sm(k) * s->num_sms));
     cudaStream_t ks = L.kstream[k];
     FF_CUDA(cudaStreamWaitEvent(ks, L.fork_ev, 0));
-    int rc = L.precision == FF_FP64 ? batch_pass_launch<double>(k, L.desc, L.maps, wl, blocks, batch_budget(k), ks)
-                                    : batch_pass_launch<float>(k, L.desc, L.maps, wl, blocks, batch_budget(k), ks);
+    int rc = L.precision == FF_FP64 ? batch_pass_launch<double>(k, L.desc, L.maps, wl, tiles, smem[k], ks)
+                                    : batch_pass_launch<float>(k, L.desc, L.maps, wl, tiles, smem[k], ks);
     if (rc != FF_OK) return rc;
     FF_CUDA(cudaEventRecord(L.kev[k], ks));
     FF_CUDA(cudaStreamWaitEvent(L.stream, L.kev[k], 0));

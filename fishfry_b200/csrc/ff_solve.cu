@@ -512,7 +512,8 @@ template <typename T> static int configure(ff_plan *p) {
       rc = p->gen[d] ? gen_prepare<T>(k, sh.smem) : bs_prepare<T>(k, sh.smem);
     if (rc != FF_OK) return rc;
     auto fill = [&](auto &g) {
-      gen_stages(L, radix, split ? gen_pad(L, radix) : 0, sh.threads, sh.units, &g.ax.S, g.ax.st);
+      if (split && sizeof(T) == 4) gen_line_stages(L, radix, gen_pad(L, radix), sh.threads, false, &g.ax.S, g.ax.st);
+      else gen_stages(L, radix, split ? gen_pad(L, radix) : 0, sh.threads, sh.units, &g.ax.S, g.ax.st);
       g.ni = ni;
       g.nj = nj;
       g.nk = nk;

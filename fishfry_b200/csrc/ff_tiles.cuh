@@ -14,7 +14,6 @@ template <typename T> struct PassArgs {
   using C = typename Cplx<T>::type;
   int ni, nj, nk, nh, nhp;
   AxisDev<C> ax[3];        // 0: x (n = ni), 1: y (nj), 2: z (nk)
-  const double *kk[3];     // (min(i, n-i) * dd)^2 per axis; kk[2] indexed by kh
   double invN;             // 1 / (ni*nj*nk)
   double dd[3];            // wavenumber scales (ParisPencil.cpp:9-11)
   int *status;             // device status word (kDev*), 0 = ok
@@ -447,33 +446,6 @@ __device__ __forceinline__ bool z_inv_tile(const typename Cplx<T>::type *spec, T
       if (la + 1 < lend) out[(la + 1) * nk + t] = v.y;
     }
     return true;
-  }
-}
-
-// The last DIF stage of the x forward transform, the filter and the first
-// DIT stage of the inverse act on the same register group.
-template <int R, int W, int NT, int NC, typename C, typename LD, typename ST, typename FL>
-__device__ __forceinline__ void fused_filter_stage(int n_rt, LD &ld, ST &st, FL &filt) {
-  const int n = NC ? NC : n_rt;
-  auto body = [&](int it) {
-    const int c = it % W;
-    const int base = (it / W) * R;
-    C v[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) v[r] = ld(base + r, c);
-    Dft<R, false, C>::run(v);
-#pragma unroll
-    for (int r = 0; r < R; r++) v[r] = filt(base + r, c, v[r]);
-    Dft<R, true, C>::run(v);
-#pragma unroll
-    for (int r = 0; r < R; r++) st(base + r, c, v[r]);
-  };
-  if constexpr (NC > 0 && (W * (NC / R)) % NT == 0) {
-    constexpr int ITER = W * (NC / R) / NT;
-#pragma unroll
-    for (int q = 0; q < ITER; q++) body((int)threadIdx.x + q * NT);
-  } else {
-    for (int it = threadIdx.x; it < W * (n / R); it += NT) body(it);
   }
 }
 

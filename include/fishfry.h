@@ -149,7 +149,7 @@ int ff_plan_destroy(ff_plan *plan);
  * physical bounds as ParisPencil's constructor takes them
  * (ParisPencil.hpp:23), or NULL for the reference's domain [-pi, pi - 2pi/n].
  * A solve of the batch runs the same five passes as ff_solve, each pass one
- * persistent kernel launch over the tiles of all grids whose axes are
+ * kernel launch over the tiles of all grids whose axes are
  * 2^a 3^b 5^c 7^d and at most 574 points, the five launches captured once
  * into a CUDA graph and replayed.  Every other grid (an axis with a prime
  * factor above 7, or longer than the batch tiles hold) is solved by its own
@@ -203,7 +203,7 @@ int ff_batch_destroy(ff_batch *batch);
  * library thread takes solves of mixed sizes and precisions as they arrive,
  * admits them against an HBM budget, and runs them with continuous batching:
  * every scheduling step carries each admitted request one pass further, all
- * requests at the same pass sharing one persistent launch (the batch
+ * requests at the same pass sharing one launch (the batch
  * kernels), so requests that arrive while others run join the next step.
  * Axis tables stay resident per (length, precision); the device memory of
  * the requests' buffers is one arena of hbm_budget bytes reserved at
