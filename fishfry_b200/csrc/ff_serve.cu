@@ -134,7 +134,7 @@ struct Lane {
   cudaEvent_t ring_ev[kRing] = {};
   long ring_step[kRing] = {-1, -1, -1};    // step occupying each ring slot (-1: free)
   long next_step = 0;
-  std::vector<uint64_t> step_members[kRing];
+  std::vector<Request *> step_members[kRing];
 };
 
 struct AxisEntry {
@@ -160,7 +160,7 @@ struct ff_server {
   std::map<std::tuple<int, int, int>, AxisEntry> axes;   // (n, precision, radix order)
   std::map<uint64_t, Request> reqs;
   std::deque<uint64_t> pending;
-  std::vector<uint64_t> active;   // admitted, not yet done (loading or running)
+  std::vector<Request *> active;  // admitted, not yet done (loading or running); the scheduler's own
   std::deque<uint64_t> finished;  // done, not yet claimed by ff_server_next
   bool admit_dirty = false;       // memory or slots freed, or requests arrived, since the last admission pass
   std::mutex mu;
@@ -257,13 +257,47 @@ void fail(ff_server *s, int rc) {
   }
 }
 
+// Device work of an admitted request: its descriptor's host image, the tables
+// of its axes, and the copy of its field into the arena.
+int start_request(ff_server *s, Request &q) {
+  batch_grid_init(q.g, q.n, nullptr, nullptr, q.precision);
+  for (int k = 0; k < 5; k++) q.g.shape[k] = batch_shape_for(q.precision, q.g, k);
+  // axis d's tables in the radix order of the pass that owns it (z: 0, y: 1, x: 2)
+  static const int owner[3] = {2, 1, 0};
+  for (int d = 0; d < 3; d++) {
+    AxisEntry *ax = nullptr;
+    int rc = axis_for(s, q.n[d], q.precision, q.g.shape[owner[d]].order, &ax);
+    if (rc != FF_OK) return rc;
+    q.g.axd[d] = ax->ad;
+    q.g.axf[d] = ax->af;
+  }
+  q.g.status = s->status;
+  q.g.density = s->arena_base + q.off_d;
+  q.g.potential = s->arena_base + q.off_p;
+  const size_t esz = q.precision == FF_FP64 ? 8 : 4;
+  const size_t fbytes = (size_t)q.n[0] * q.n[1] * q.n[2] * esz;
+  // the copy stream does not synchronise with the legacy default stream:
+  // the input copy waits explicitly for the work queued there before the
+  // submission (a field produced by the caller on that stream)
+  FF_CUDA(cudaStreamWaitEvent(s->copy, q.src_ev, 0));
+  FF_CUDA(cudaMemcpyAsync(q.g.density, q.f, fbytes, q.f_on_host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice,
+                          s->copy));
+  if (!q.in_ev) FF_CUDA(cudaEventCreateWithFlags(&q.in_ev, cudaEventDisableTiming));
+  FF_CUDA(cudaEventRecord(q.in_ev, s->copy));
+  return FF_OK;
+}
+
 // Admission of pending requests in arrival order; a request that does not
 // fit now is passed over (later, smaller ones may fit) and retried when
 // memory or slots are freed.  At most kAdmitWindow queued requests are
 // examined per pass, so a long queue costs nothing while the budget is full.
 constexpr int kAdmitWindow = 64;
 
-int admit(ff_server *s) {
+// The bookkeeping runs under the caller's lock; the device work (tables, input
+// copies) runs with it released, so that submissions and fetches do not queue
+// behind it: other threads leave a request alone once it is past kPending.
+int admit(ff_server *s, std::unique_lock<std::mutex> &lk) {
+  std::vector<Request *> fresh;
   int seen = 0;
   for (auto it = s->pending.begin(); it != s->pending.end() && seen < kAdmitWindow; seen++) {
     Request &q = s->reqs[*it];
@@ -286,59 +320,30 @@ int admit(ff_server *s) {
     q.off_p = op;
     q.slot = L.free_slots.back();
     L.free_slots.pop_back();
-    batch_grid_init(q.g, q.n, nullptr, nullptr, q.precision);
-    for (int k = 0; k < 5; k++) q.g.shape[k] = batch_shape_for(q.precision, q.g, k);
-    // axis d's tables in the radix order of the pass that owns it (z: 0, y: 1, x: 2)
-    static const int owner[3] = {2, 1, 0};
-    for (int d = 0; d < 3; d++) {
-      AxisEntry *ax = nullptr;
-      int rc = axis_for(s, q.n[d], q.precision, q.g.shape[owner[d]].order, &ax);
-      if (rc != FF_OK) return rc;
-      q.g.axd[d] = ax->ad;
-      q.g.axf[d] = ax->af;
-    }
-    q.g.status = s->status;
-    q.g.density = s->arena_base + q.off_d;
-    q.g.potential = s->arena_base + q.off_p;
-    const size_t esz = q.precision == FF_FP64 ? 8 : 4;
-    const size_t fbytes = (size_t)q.n[0] * q.n[1] * q.n[2] * esz;
-    // the copy stream does not synchronise with the legacy default stream:
-    // the input copy waits explicitly for the work queued there before the
-    // submission (a field produced by the caller on that stream)
-    FF_CUDA(cudaStreamWaitEvent(s->copy, q.src_ev, 0));
-    FF_CUDA(cudaMemcpyAsync(q.g.density, q.f, fbytes, q.f_on_host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice,
-                            s->copy));
-    if (!q.in_ev) FF_CUDA(cudaEventCreateWithFlags(&q.in_ev, cudaEventDisableTiming));
-    FF_CUDA(cudaEventRecord(q.in_ev, s->copy));
     q.state = kLoading;
     q.t_admit = Clock::now();
-    s->active.push_back(q.id);
+    s->active.push_back(&q);
+    fresh.push_back(&q);
     it = s->pending.erase(it);
   }
-  return FF_OK;
+  if (fresh.empty()) return FF_OK;
+  lk.unlock();
+  int rc = FF_OK;
+  for (Request *q : fresh) {
+    rc = start_request(s, *q);
+    if (rc != FF_OK) break;
+  }
+  lk.lock();
+  return rc;
 }
 
-// Builds and launches the next step of one precision lane; returns whether
-// a step was issued.
-int issue_step(ff_server *s, Lane &L, bool *issued) {
-  *issued = false;
-  int r = -1;
-  for (int q = 0; q < kRing; q++)
-    if (L.ring_step[q] < 0) {
-      r = q;
-      break;
-    }
-  if (r < 0) return FF_OK;
-  std::vector<uint64_t> members;
-  for (uint64_t id : s->active) {
-    Request &q = s->reqs[id];
-    if (q.state == kRunning && q.precision == L.precision && q.next_pass < 5) members.push_back(q.id);
-  }
-  if (members.empty()) return FF_OK;
+// The device work of a step: its members' new descriptors, its work lists and
+// its launches, in ring block r.
+int launch_step(ff_server *s, Lane &L, int r, const std::vector<Request *> &members, int *launches) {
   // compact layout of this step's work lists in ring block r: per kind the
   // entries (int2) and the prefix sums (int)
   int cnt[5] = {0, 0, 0, 0, 0};
-  for (uint64_t id : members) cnt[s->reqs[id].next_pass]++;
+  for (const Request *q : members) cnt[q->next_pass]++;
   size_t e_off[5], s_off[5], off = 0;
   for (int k = 0; k < 5; k++) {
     e_off[k] = off;
@@ -351,19 +356,17 @@ int issue_step(ff_server *s, Lane &L, bool *issued) {
   int fill[5] = {0, 0, 0, 0, 0};
   size_t smem[5] = {0, 0, 0, 0, 0};
   for (int k = 0; k < 5; k++) reinterpret_cast<int *>(hb + s_off[k])[0] = 0;
-  for (uint64_t id : members) {
-    Request &q = s->reqs[id];
+  std::vector<int> fresh;   // slots whose descriptors are new
+  for (Request *m : members) {
+    Request &q = *m;
     if (!q.desc_uploaded) {
       unsigned char *img = L.desc_host + (size_t)q.slot * L.dsz;
       if (L.precision == FF_FP64) batch_desc_fill<double>(img, q.g);
       else batch_desc_fill<float>(img, q.g);
-      FF_CUDA(cudaMemcpyAsync(static_cast<char *>(L.desc) + (size_t)q.slot * L.dsz, img, L.dsz,
-                              cudaMemcpyHostToDevice, L.stream));
       CUtensorMap *mh = L.maps_host + 2 * (size_t)q.slot;
       const int rc = batch_grid_maps(q.g, q.precision, mh);
       if (rc != FF_OK) return rc;
-      FF_CUDA(cudaMemcpyAsync(L.maps + 2 * (size_t)q.slot, mh, 2 * sizeof(CUtensorMap), cudaMemcpyHostToDevice,
-                              L.stream));
+      fresh.push_back(q.slot);
       q.desc_uploaded = true;
     }
     const int k = q.next_pass;
@@ -375,23 +378,64 @@ int issue_step(ff_server *s, Lane &L, bool *issued) {
     q.next_pass++;
     if (q.next_pass == 5) q.finish_step = L.next_step;
   }
+  // one copy per run of neighbouring slots
+  std::sort(fresh.begin(), fresh.end());
+  for (size_t i = 0, j; i < fresh.size(); i = j) {
+    for (j = i + 1; j < fresh.size() && fresh[j] == fresh[j - 1] + 1;) j++;
+    const size_t first = fresh[i], count = j - i;
+    FF_CUDA(cudaMemcpyAsync(static_cast<char *>(L.desc) + first * L.dsz, L.desc_host + first * L.dsz, count * L.dsz,
+                            cudaMemcpyHostToDevice, L.stream));
+    FF_CUDA(cudaMemcpyAsync(L.maps + 2 * first, L.maps_host + 2 * first, 2 * count * sizeof(CUtensorMap),
+                            cudaMemcpyHostToDevice, L.stream));
+  }
   FF_CUDA(cudaMemcpyAsync(db, hb, off, cudaMemcpyHostToDevice, L.stream));
-  FF_CUDA(cudaEventRecord(L.fork_ev, L.stream));
+  // a step of one kind runs on the lane's stream; the kinds of a mixed step fork
+  // from it and join it
+  int kinds = 0;
+  for (int k = 0; k < 5; k++) kinds += cnt[k] > 0;
+  if (kinds > 1) FF_CUDA(cudaEventRecord(L.fork_ev, L.stream));
   for (int k = 0; k < 5; k++) {
     if (!cnt[k]) continue;
     const BatchWork wl{reinterpret_cast<const int2 *>(db + e_off[k]), reinterpret_cast<const int *>(db + s_off[k]),
                        cnt[k], batch_blocks_per_sm(k) * s->num_sms};
     const int tiles = reinterpret_cast<int *>(hb + s_off[k])[cnt[k]];
-    cudaStream_t ks = L.kstream[k];
-    FF_CUDA(cudaStreamWaitEvent(ks, L.fork_ev, 0));
+    cudaStream_t ks = kinds > 1 ? L.kstream[k] : L.stream;
+    if (kinds > 1) FF_CUDA(cudaStreamWaitEvent(ks, L.fork_ev, 0));
     int rc = L.precision == FF_FP64 ? batch_pass_launch<double>(k, L.desc, L.maps, wl, tiles, smem[k], ks)
                                     : batch_pass_launch<float>(k, L.desc, L.maps, wl, tiles, smem[k], ks);
     if (rc != FF_OK) return rc;
-    FF_CUDA(cudaEventRecord(L.kev[k], ks));
-    FF_CUDA(cudaStreamWaitEvent(L.stream, L.kev[k], 0));
-    s->launches++;
+    if (kinds > 1) {
+      FF_CUDA(cudaEventRecord(L.kev[k], ks));
+      FF_CUDA(cudaStreamWaitEvent(L.stream, L.kev[k], 0));
+    }
+    (*launches)++;
   }
   FF_CUDA(cudaEventRecord(L.ring_ev[r], L.stream));
+  return FF_OK;
+}
+
+// Builds and launches the next step of one precision lane; returns whether
+// a step was issued.  Touches only what the scheduler owns (members on the
+// device, the lane's ring), so the caller's lock is released meanwhile.
+int issue_step(ff_server *s, Lane &L, std::unique_lock<std::mutex> &lk, bool *issued) {
+  *issued = false;
+  int r = -1;
+  for (int q = 0; q < kRing; q++)
+    if (L.ring_step[q] < 0) {
+      r = q;
+      break;
+    }
+  if (r < 0) return FF_OK;
+  std::vector<Request *> members;
+  for (Request *q : s->active)
+    if (q->state == kRunning && q->precision == L.precision && q->next_pass < 5) members.push_back(q);
+  if (members.empty()) return FF_OK;
+  int launches = 0;
+  lk.unlock();
+  const int rc = launch_step(s, L, r, members, &launches);
+  lk.lock();
+  s->launches += launches;
+  if (rc != FF_OK) return rc;
   L.ring_step[r] = L.next_step++;
   L.step_members[r] = members;
   s->steps++;
@@ -415,15 +459,13 @@ int retire_steps(ff_server *s, Lane &L, bool *progress) {
     if (e == cudaErrorNotReady) return FF_OK;
     if (e != cudaSuccess) FF_CUDA(e);
     const auto now = Clock::now();
-    for (uint64_t id : L.step_members[r]) {
-      auto it = s->reqs.find(id);
-      if (it == s->reqs.end()) continue;
-      Request &q = it->second;
+    for (Request *m : L.step_members[r]) {
+      Request &q = *m;
       if (q.finish_step == oldest && q.state == kRunning) {
-        s->active.erase(std::find(s->active.begin(), s->active.end(), id));
+        s->active.erase(std::find(s->active.begin(), s->active.end(), m));
         q.state = kDone;
         q.t_done = now;
-        s->finished.push_back(id);
+        s->finished.push_back(q.id);
         s->completed++;
         s->lat_ms.push_back(ms_between(q.t_submit, q.t_done));
         s->points_done += double(q.n[0]) * q.n[1] * q.n[2];
@@ -446,11 +488,11 @@ void scheduler(ff_server *s) {
     if (progress) s->cv_done.notify_all();
     if (rc == FF_OK && !s->pending.empty() && s->admit_dirty) {
       s->admit_dirty = false;
-      rc = admit(s);
+      rc = admit(s, lk);
     }
     if (rc == FF_OK) {
-      for (uint64_t id : s->active) {
-        Request &q = s->reqs[id];
+      for (Request *m : s->active) {
+        Request &q = *m;
         if (q.state != kLoading) continue;
         const cudaError_t e = cudaEventQuery(q.in_ev);
         if (e == cudaSuccess) {
@@ -464,7 +506,7 @@ void scheduler(ff_server *s) {
     }
     for (int l = 0; l < 2 && rc == FF_OK; l++) {
       bool issued = false;
-      rc = issue_step(s, s->lane[l], &issued);
+      rc = issue_step(s, s->lane[l], lk, &issued);
       progress = progress || issued;
     }
     const bool busy = !s->active.empty();
