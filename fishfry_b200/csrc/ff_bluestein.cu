@@ -24,6 +24,7 @@
 
 #include "ff_bluestein.hpp"
 #include "ff_gen_stages.cuh"
+#include "ff_launch.hpp"
 
 namespace ff {
 
@@ -99,6 +100,8 @@ __global__ void __launch_bounds__(256, 3)
     mbar_init(&mbar, 1);
     mbar_init_fence();
   }
+  pdl_start();
+  pdl_wait();
   __syncthreads();
   lines_in(a, raw, f, line0, nl, &mbar);
   if (!z_wait(&mbar, a.status, a.wait_iters)) return;
@@ -172,6 +175,7 @@ __global__ void __launch_bounds__(256, 3)
     mbar_init(&mbar, 1);
     mbar_init_fence();
   }
+  pdl_wait();
   __syncthreads();
   rows_in(stage, a.sp * sizeof(C), reinterpret_cast<const unsigned char *>(spec + line0 * a.nhp), a.nhp * sizeof(C), nl,
           &mbar);
@@ -236,6 +240,8 @@ __global__ void __launch_bounds__(256, 3)
   constexpr int CU = 16 / sizeof(C);
   extern __shared__ unsigned char smraw[];
   V *tile = reinterpret_cast<V *>(align128(smraw));
+  pdl_start();
+  pdl_wait();
   const int n = a.n;
   const int W = CU << a.lu;
   const int ktiles = (a.nh + W - 1) / W;
@@ -413,17 +419,18 @@ template <typename T>
 int bs_launch(int kind, const BsPass<typename Cplx<T>::type> &a, const GenShape &s, const void *in, void *out,
               cudaStream_t st) {
   using C = typename Cplx<T>::type;
-  const unsigned grid = (unsigned)s.grid;
   const C *ci = static_cast<const C *>(in);
   C *co = static_cast<C *>(out);
+  auto go = [&](auto k, auto... args) { return launch_chained(s.chained, k, (unsigned)s.grid, s.threads, s.smem, st, args...); };
+  cudaError_t e;
   switch (kind) {
-    case 0: k_bs_zfwd<T><<<grid, s.threads, s.smem, st>>>(static_cast<const T *>(in), co, a); break;
-    case 1: k_bs_strided<T, 1><<<grid, s.threads, s.smem, st>>>(ci, co, a); break;
-    case 2: k_bs_strided<T, 2><<<grid, s.threads, s.smem, st>>>(ci, co, a); break;
-    case 3: k_bs_strided<T, 3><<<grid, s.threads, s.smem, st>>>(ci, co, a); break;
-    default: k_bs_zinv<T><<<grid, s.threads, s.smem, st>>>(ci, static_cast<T *>(out), a); break;
+    case 0: e = go(k_bs_zfwd<T>, static_cast<const T *>(in), co, a); break;
+    case 1: e = go(k_bs_strided<T, 1>, ci, co, a); break;
+    case 2: e = go(k_bs_strided<T, 2>, ci, co, a); break;
+    case 3: e = go(k_bs_strided<T, 3>, ci, co, a); break;
+    default: e = go(k_bs_zinv<T>, ci, static_cast<T *>(out), a); break;
   }
-  FF_CUDA(cudaGetLastError());
+  FF_CUDA(e);
   return FF_OK;
 }
 

@@ -872,6 +872,12 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
 }
 
+// Programmatic dependent launch (launch_chained): lets the dependent kernel's
+// blocks start once every block of this one has called it; waits for the
+// completion of the kernels this one depends on (no effect on other launches).
+__device__ __forceinline__ void pdl_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Device-side status word values (plan status buffer).
 enum : int { kDevOk = 0, kDevTmaTimeout = 1, kDevDepTimeout = 2 };
 

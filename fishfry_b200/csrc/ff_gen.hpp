@@ -77,6 +77,7 @@ struct GenShape {
   int threads;
   size_t smem;
   long grid;
+  bool chained;   // launched as a programmatic dependent (ff_launch.hpp)
   int box_rows;   // strided passes: rows per TMA box
   int tile_rows;  // z passes
   int lp, sp;     // z passes: pitch of a staged real line (values), of a staged spectrum row (complex values)

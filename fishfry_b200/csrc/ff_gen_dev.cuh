@@ -32,6 +32,7 @@
 #pragma once
 
 #include "ff_gen_lines.cuh"
+#include "ff_launch.hpp"
 
 namespace ff {
 
@@ -122,6 +123,8 @@ __global__ void __launch_bounds__(256, 3)
   const int ktiles = (a.nh + W - 1) / W;
   const int o = blockIdx.x / ktiles, kt = blockIdx.x - o * ktiles;
   const int rows = a.box_rows;
+  pdl_start();
+  pdl_wait();
   if (threadIdx.x == 0) {
     mbar_init(&mbar, 1);
     mbar_init_fence();
@@ -181,6 +184,8 @@ __global__ void __launch_bounds__(256, 3)
   // rows in and out, in bytes
   const size_t rin = KIND == 0 ? a.nk * sizeof(float) : a.nhp * sizeof(float2);
   const unsigned char *src = static_cast<const unsigned char *>(in);
+  if (KIND == 0) pdl_start();
+  pdl_wait();
   if (threadIdx.x == 0) {
     mbar_init(&mbar, 1);
     mbar_init_fence();
@@ -227,6 +232,8 @@ __global__ void __launch_bounds__(256, 3)
     mbar_init(&mbar, 1);
     mbar_init_fence();
   }
+  pdl_start();
+  pdl_wait();
   __syncthreads();
   lines_in(a, raw, f, line0, nl, &mbar);
   if (threadIdx.x == blockDim.x - 1 && a.l2_ahead > 0) {
@@ -329,6 +336,7 @@ __global__ void __launch_bounds__(256, 3)
     mbar_init(&mbar, 1);
     mbar_init_fence();
   }
+  pdl_wait();
   __syncthreads();
   rows_in(stage, a.sp * sizeof(C), reinterpret_cast<const unsigned char *>(spec + line0 * a.nhp), a.nhp * sizeof(C), nl,
           &mbar);
@@ -420,21 +428,22 @@ template <typename T>
 int gen_launch(int kind, const GenPass<typename Cplx<T>::type> &a, const GenShape &s, const CUtensorMap *map,
                const void *in, void *out, cudaStream_t st) {
   using C = typename Cplx<T>::type;
-  const unsigned grid = (unsigned)s.grid;
+  auto go = [&](auto k, auto... args) { return launch_chained(s.chained, k, (unsigned)s.grid, s.threads, s.smem, st, args...); };
+  cudaError_t e;
   switch (kind) {
     case 0:
-      if constexpr (sizeof(T) == 4) k_gen_lines<0><<<grid, s.threads, s.smem, st>>>(in, out, a);
-      else k_gen_zfwd<T><<<grid, s.threads, s.smem, st>>>(static_cast<const T *>(in), static_cast<C *>(out), a);
+      if constexpr (sizeof(T) == 4) e = go(k_gen_lines<0>, in, out, a);
+      else e = go(k_gen_zfwd<T>, static_cast<const T *>(in), static_cast<C *>(out), a);
       break;
-    case 1: k_gen_strided<T, 1><<<grid, s.threads, s.smem, st>>>(*map, static_cast<C *>(out), a); break;
-    case 2: k_gen_strided<T, 2><<<grid, s.threads, s.smem, st>>>(*map, static_cast<C *>(out), a); break;
-    case 3: k_gen_strided<T, 3><<<grid, s.threads, s.smem, st>>>(*map, static_cast<C *>(out), a); break;
+    case 1: e = go(k_gen_strided<T, 1>, *map, static_cast<C *>(out), a); break;
+    case 2: e = go(k_gen_strided<T, 2>, *map, static_cast<C *>(out), a); break;
+    case 3: e = go(k_gen_strided<T, 3>, *map, static_cast<C *>(out), a); break;
     default:
-      if constexpr (sizeof(T) == 4) k_gen_lines<4><<<grid, s.threads, s.smem, st>>>(in, out, a);
-      else k_gen_zinv<T><<<grid, s.threads, s.smem, st>>>(static_cast<const C *>(in), static_cast<T *>(out), a);
+      if constexpr (sizeof(T) == 4) e = go(k_gen_lines<4>, in, out, a);
+      else e = go(k_gen_zinv<T>, static_cast<const C *>(in), static_cast<T *>(out), a);
       break;
   }
-  FF_CUDA(cudaGetLastError());
+  FF_CUDA(e);
   return FF_OK;
 }
 

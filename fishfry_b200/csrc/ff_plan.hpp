@@ -51,6 +51,7 @@ struct ff_plan {
   int zW, zP;          // z passes: line pairs per block, line pitch in complex values
   size_t zsmem;
   unsigned ztiles;
+  bool chained;        // passes as programmatic dependents of one another (ff_launch.hpp)
   int l2_ahead;        // forward z pass: L2 prefetch distance in blocks (0: off)
   int wait_iters;      // bounded device waits: iteration limit of the first wait (0: built-in)
   int dep_extra;       // fused passes: added to every dependency wait's target (test hook, 0)

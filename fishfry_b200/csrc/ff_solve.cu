@@ -28,6 +28,7 @@
 
 #include "ff_bluestein.hpp"
 #include "ff_fft.cuh"
+#include "ff_launch.hpp"
 #include "ff_plan.hpp"
 #include "ff_status.hpp"
 #include "ff_tiles.cuh"
@@ -59,6 +60,8 @@ __global__ void __launch_bounds__(kZPassThreads, 6) k_zfwd(const T *__restrict__
     mbar_init(&mbar, 1);
     mbar_init_fence();
   }
+  pdl_start();
+  pdl_wait();
   __syncthreads();
   const long nlines = (long)a.ni * a.nj;
   if (threadIdx.x == 0) {
@@ -81,6 +84,7 @@ __global__ void __launch_bounds__(kZPassThreads, 6) k_zinv(const typename Cplx<T
     mbar_init(&mbar, 1);
     mbar_init_fence();
   }
+  pdl_wait();
   __syncthreads();
   const long nlines = (long)a.ni * a.nj;
   // the same L2 hint as the forward pass, on the spectrum rows (contiguous
@@ -114,6 +118,8 @@ __global__ void __launch_bounds__(kZThreads, 3)
     mbar_init(&mbar, 1);
     mbar_init_fence();
   }
+  pdl_start();
+  pdl_wait();
   __syncthreads();
   if (!tma_tile<C, W, XPASS>(&tmap, sm, &mbar, 0, n, box_rows, o, kt, a.status, a.wait_iters)) return;
   if (XPASS) {
@@ -508,6 +514,7 @@ template <typename T> static int configure(ff_plan *p) {
         ? gen_shape(kind, ni, nj, nk, p->nhp, (int)sizeof(T), radix, p->num_sms)
         : bs_shape(kind, ni, nj, nk, p->nhp, (int)sizeof(T), L, p->num_sms);
     p->gshape[d] = sh;
+    p->gshape[d].chained = p->chained;
     for (int k = kind; k <= 4 && rc == FF_OK; k = k == 0 ? 4 : k == 1 ? 3 : 5)
       rc = p->gen[d] ? gen_prepare<T>(k, sh.smem) : bs_prepare<T>(k, sh.smem);
     if (rc != FF_OK) return rc;
@@ -647,9 +654,8 @@ static int launch_strided(const ff_plan *p, int kind, const CUtensorMap &map, co
   if (p->bsM[axis]) return bs_launch<T>(kind, bs_pass<T>(p, axis), p->gshape[axis], src, dst, st);
   if (p->gen[axis]) return gen_launch<T>(kind, gen_pass<T>(p, axis), p->gshape[axis], &map, nullptr, dst, st);
   const StridedCfg &cfg = axis == 0 ? p->xcfg : p->ycfg;
-  strided_kernel<T>(kind == 1 ? 0 : kind == 3 ? 1 : 2, cfg.N)<<<cfg.grid, kZThreads, cfg.smem, st>>>(
-      map, dst, a, cfg.box_rows);
-  FF_CUDA(cudaGetLastError());
+  FF_CUDA(launch_chained(p->chained, strided_kernel<T>(kind == 1 ? 0 : kind == 3 ? 1 : 2, cfg.N), cfg.grid, kZThreads, cfg.smem, st,
+                         map, dst, a, cfg.box_rows));
   return FF_OK;
 }
 
@@ -660,12 +666,11 @@ template <typename T> static int launch_z(const ff_plan *p, bool inverse, void *
   if (p->gen[2])
     return gen_launch<T>(inverse ? 4 : 0, gen_pass<T>(p, 2), p->gshape[2], nullptr, in, out, st);
   if (!inverse)
-    zfwd_kernel<T>(p->zN)<<<p->ztiles, kZPassThreads, p->zsmem, st>>>(static_cast<const T *>(in),
-                                                                          static_cast<C *>(out), a, p->zW, p->zP);
+    FF_CUDA(launch_chained(p->chained, zfwd_kernel<T>(p->zN), p->ztiles, kZPassThreads, p->zsmem, st, static_cast<const T *>(in),
+                           static_cast<C *>(out), a, p->zW, p->zP));
   else
-    zinv_kernel<T>(p->zN)<<<p->ztiles, kZPassThreads, p->zsmem, st>>>(static_cast<const C *>(in),
-                                                                          static_cast<T *>(out), a, p->zW, p->zP);
-  FF_CUDA(cudaGetLastError());
+    FF_CUDA(launch_chained(p->chained, zinv_kernel<T>(p->zN), p->ztiles, kZPassThreads, p->zsmem, st, static_cast<const C *>(in),
+                           static_cast<T *>(out), a, p->zW, p->zP));
   return FF_OK;
 }
 
@@ -822,6 +827,7 @@ int ff_plan_create(const int n[3], const double lo[3], const double hi[3], int p
   const size_t spec = (size_t)n[0] * n[1] * p->nhp * csz;
   const size_t real = (size_t)n[0] * n[1] * n[2] * (csz / 2);
   p->bytes = std::max(spec, real);
+  p->chained = spec <= kChainBytes;
   if (cudaGetDevice(&p->device) != cudaSuccess ||
       cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device) != cudaSuccess) {
     delete p;

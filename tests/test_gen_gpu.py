@@ -96,3 +96,47 @@ def test_lengths_with_larger_prime_factors(torch_cuda, ff, axis, precision):
 @pytest.mark.parametrize("n", [(100, 90, 81), (96, 75, 80), (147, 98, 105), (200, 180, 160)])
 def test_grids_of_several_waves(torch_cuda, ff, n, precision):
     check(torch_cuda, ff, n, precision)
+
+
+# Passes launched as programmatic dependents of one another: results of solves
+# queued back to back on shared buffers, on the default and a side stream, and
+# replayed from a captured graph.
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("n", [(64, 64, 64), (30, 45, 50), (33, 34, 35)])
+def test_chained_passes_back_to_back_and_captured(torch_cuda, ff, n, precision):
+    torch = torch_cuda
+    dt = torch.float64 if precision == 0 else torch.float32
+    plan = ff.Plan(n, precision=precision)
+    size, N = plan.nbytes // (8 if precision == 0 else 4), n[0] * n[1] * n[2]
+    fields = [torch.randn(N, dtype=dt, device="cuda") for _ in range(4)]
+    d, p = (torch.zeros(size, dtype=dt, device="cuda") for _ in range(2))
+    want = []
+    for f in fields:
+        d[:N] = f
+        torch.cuda.synchronize()
+        plan.solve(d, p)
+        torch.cuda.synchronize()
+        want.append(p[:N].clone())
+
+    def run(stream):
+        out = []
+        for f in fields:
+            d[:N].copy_(f)
+            plan.solve(d, p, stream=stream)
+            out.append(p[:N].clone())
+        return out
+
+    side = torch.cuda.Stream()
+    got = run(None)
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        got += run(side)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = run(torch.cuda.current_stream())
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    for q, out in enumerate(got + captured):
+        assert torch.equal(out, want[q % len(fields)]), q
