@@ -222,14 +222,9 @@ void gen_pick_threads(GenShape *s) {
   s->threads = std::min(256, std::max(64, 768 / blocks / 32 * 32));
 }
 
-void gen_z_shape(GenShape *s, int ni, int nj, int nk, int nhp, int esz, int num_sms, bool lines_kind) {
+void gen_z_shape(GenShape *s, int ni, int nj, int nk, int nhp, int esz, int num_sms, bool lines_kind, size_t limit) {
   const int cu = 16 / (2 * esz);   // line pairs per unit
   const long nlines = (long)ni * nj;
-  // many small tiles (up to 40 KB, five or more blocks on an SM) beat fewer
-  // large ones for short lines and tie for long ones: 200x180x160 FP32 z
-  // 20.9 / 21.5 us against 26.2 / 23.5 at 56 KB, 500^3 FP64 425 / 431 against
-  // 443 / 455 at 74 KB
-  const size_t limit = 40 * 1024;
   for (s->units = 8;; s->units /= 2) {
     const int lines = 2 * cu * s->units;
     // pitches that put neighbouring units' lines and rows in different banks
@@ -254,7 +249,11 @@ GenShape gen_shape(int kind, int ni, int nj, int nk, int nhp, int esz, const std
   const int cu = 16 / (2 * esz);   // complex columns (or line pairs) per unit
   if (kind == 0 || kind == 4) {
     s.tile_rows = nk + gen_pad(nk, radix) * (radix[0] - 1);
-    gen_z_shape(&s, ni, nj, nk, nhp, esz, num_sms, esz == 4);
+    // many small tiles (up to 40 KB, five or more blocks on an SM) beat fewer
+    // large ones for short lines and tie for long ones: 200x180x160 FP32 z
+    // 20.9 / 21.5 us against 26.2 / 23.5 at 56 KB, 500^3 FP64 425 / 431 against
+    // 443 / 455 at 74 KB
+    gen_z_shape(&s, ni, nj, nk, nhp, esz, num_sms, esz == 4, 40 * 1024);
     return s;
   }
   const int n = kind == 2 ? ni : nj;

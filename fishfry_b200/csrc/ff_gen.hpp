@@ -89,8 +89,9 @@ GenShape gen_shape(int kind, int ni, int nj, int nk, int nhp, int esz, const std
 
 // Parts of gen_shape that other tiles share: units, pitches, shared memory and
 // grid of a z pass whose tile has s->tile_rows rows (lines_kind: a tile with
-// butterflies fastest); threads per block from the shared memory.
-void gen_z_shape(GenShape *s, int ni, int nj, int nk, int nhp, int esz, int num_sms, bool lines_kind);
+// butterflies fastest), the most units that keep `limit` bytes of shared memory;
+// threads per block from the shared memory.
+void gen_z_shape(GenShape *s, int ni, int nj, int nk, int nhp, int esz, int num_sms, bool lines_kind, size_t limit);
 void gen_pick_threads(GenShape *s);
 
 // Cost of an n-point transform's stages per point (arbitrary unit).

@@ -57,9 +57,11 @@ struct ff_plan {
   int dep_extra;       // fused passes: added to every dependency wait's target (test hook, 0)
   ff::StridedCfg ycfg, xcfg;
   ff::FusedCfg fwd, inv;
-  // axes with a prime factor above 7: padded convolution length M (0 for a
-  // 2^a 3^b 5^c 7^d axis), pass arguments and launch shape by axis
+  // axes with a prime factor above 7: convolution length (0 for a
+  // 2^a 3^b 5^c 7^d axis; n - 1 where Rader's algorithm applies, else Bluestein's
+  // M), pass arguments and launch shape by axis
   int bsM[3];
+  bool rader[3];
   ff::BsPass<double2> bspd[3];
   ff::BsPass<float2> bspf[3];
   // axes of 2^a 3^b 5^c 7^d points without a compile-time plan (ff_gen_dev.cuh):

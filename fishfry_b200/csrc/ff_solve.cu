@@ -512,11 +512,14 @@ template <typename T> static int configure(ff_plan *p) {
     const std::vector<int> radix = gen_radices(L, split);
     const GenShape sh = p->gen[d]
         ? gen_shape(kind, ni, nj, nk, p->nhp, (int)sizeof(T), radix, p->num_sms)
-        : bs_shape(kind, ni, nj, nk, p->nhp, (int)sizeof(T), L, p->num_sms);
+        : bs_shape(kind, ni, nj, nk, p->nhp, (int)sizeof(T), L + p->rader[d], p->num_sms);
+    // the lengths an axis may have are those whose Bluestein tile fits
+    const size_t need = !p->rader[d] ? sh.smem
+        : bs_shape(kind, ni, nj, nk, p->nhp, (int)sizeof(T), bs_padded_length(p->n[d]), p->num_sms).smem;
     p->gshape[d] = sh;
     p->gshape[d].chained = p->chained;
     for (int k = kind; k <= 4 && rc == FF_OK; k = k == 0 ? 4 : k == 1 ? 3 : 5)
-      rc = p->gen[d] ? gen_prepare<T>(k, sh.smem) : bs_prepare<T>(k, sh.smem);
+      rc = p->gen[d] ? gen_prepare<T>(k, sh.smem) : bs_prepare<T>(k, p->rader[d], need);
     if (rc != FF_OK) return rc;
     auto fill = [&](auto &g) {
       if (split && sizeof(T) == 4) gen_line_stages(L, radix, gen_pad(L, radix), sh.threads, false, &g.ax.S, g.ax.st);
@@ -842,12 +845,24 @@ int ff_plan_create(const int n[3], const double lo[3], const double hi[3], int p
   int len[3];
   size_t off = 0;
   size_t o_tw[3], o_tw64[3], o_rev[3], o_ipos[3], o_chirp[3] = {0, 0, 0}, o_ghat[3] = {0, 0, 0};
+  std::vector<int> perm[3];
   auto take = [&](size_t b) { size_t o = off; off += (b + 255) & ~size_t(255); return o; };
   for (int d = 0; d < 3; d++) {
-    p->bsM[d] = smooth2357(n[d]) ? 0 : bs_padded_length(n[d]);
+    const int root = smooth2357(n[d]) ? 0 : rader_root(n[d]);
+    p->rader[d] = root != 0;
+    p->bsM[d] = smooth2357(n[d]) ? 0 : root ? n[d] - 1 : bs_padded_length(n[d]);
     const int L = len[d] = p->bsM[d] ? p->bsM[d] : n[d];
     if (p->bsM[d]) {
-      o_chirp[d] = take(n[d] * csz);
+      if (root) {
+        perm[d].resize(n[d] - 1);
+        long long v = 1;
+        for (int &q : perm[d]) {
+          q = (int)v;
+          v = v * root % n[d];
+        }
+      } else {
+        o_chirp[d] = take(n[d] * csz);
+      }
       o_ghat[d] = take(L * csz);
       continue;
     }
@@ -860,7 +875,7 @@ int ff_plan_create(const int n[3], const double lo[3], const double hi[3], int p
     o_tw[d] = take(L * csz);
     o_tw64[d] = precision == FF_FP64 ? o_tw[d] : take(L * sizeof(double2));
   }
-  size_t o_gen[3] = {0, 0, 0}, o_gidx[3] = {0, 0, 0};
+  size_t o_gen[3] = {0, 0, 0}, o_gidx[3] = {0, 0, 0}, o_perm[3] = {0, 0, 0};
   std::vector<int> gradix[3], gidx[3];
   for (int d = 0; d < 3; d++) {
     p->gen[d] = !p->bsM[d] && special_n(n[d]) == 0;
@@ -876,6 +891,7 @@ int ff_plan_create(const int n[3], const double lo[3], const double hi[3], int p
     o_rev[d] = take(rev[d].size() * sizeof(int));
     o_ipos[d] = take(rev[d].size() * sizeof(int));
     if (!gidx[d].empty()) o_gidx[d] = take(gidx[d].size() * sizeof(int));
+    if (!perm[d].empty()) o_perm[d] = take(perm[d].size() * sizeof(int));
   }
   const size_t int_bytes = off - o_int;
   const size_t o_status = take(sizeof(int));
@@ -907,6 +923,7 @@ int ff_plan_create(const int n[3], const double lo[3], const double hi[3], int p
         hrev[q] = rev[d][q];
         hpos[rev[d][q]] = q;
       }
+      if (!perm[d].empty()) std::memcpy(host.data() + (o_perm[d] - o_int), perm[d].data(), perm[d].size() * sizeof(int));
       if (!gidx[d].empty()) std::memcpy(host.data() + (o_gidx[d] - o_int), gidx[d].data(), gidx[d].size() * sizeof(int));
     }
     if (rc == FF_OK && cudaMemcpy(base + o_int, host.data(), int_bytes, cudaMemcpyHostToDevice) != cudaSuccess)
@@ -940,11 +957,15 @@ int ff_plan_create(const int n[3], const double lo[3], const double hi[3], int p
       auto build = [&](auto &bs) {
         using BC = std::remove_const_t<std::remove_pointer_t<decltype(bs.chirp)>>;
         BC *ch = reinterpret_cast<BC *>(base + o_chirp[d]), *gh = reinterpret_cast<BC *>(base + o_ghat[d]);
+        const int *pm = reinterpret_cast<const int *>(base + o_perm[d]);
         bs.n = n[d];
-        bs.chirp = ch;
+        bs.perm = p->rader[d] ? pm : nullptr;
+        bs.chirp = p->rader[d] ? nullptr : ch;
         bs.ghat = gh;
         const int r = gen_axis_build(L, gradix[d], base + o_gen[d], idx, &bs.ax);
-        return r == FF_OK ? bs_tables<BC>(n[d], L, idx, gradix[d].back(), ch, gh) : r;
+        if (r != FF_OK) return r;
+        return p->rader[d] ? rader_tables<BC>(n[d], pm, idx, gradix[d].back(), gh)
+                           : bs_tables<BC>(n[d], L, idx, gradix[d].back(), ch, gh);
       };
       rc = precision == FF_FP64 ? build(p->bspd[d]) : build(p->bspf[d]);
     }
