@@ -202,6 +202,44 @@ template <bool INV, typename C> struct Dft<8, INV, C> {
   }
 };
 
+// 16 = 4 x 4: r = 4 r1 + r2, s = s1 + 4 s2, factors w16^(r2 s1) between.
+// cos and sin of pi / 8
+#define FF_C16_1 0.92387953251128675612818318939678828682
+#define FF_S16_1 0.38268343236508977172845998403039886676
+template <bool INV, typename C> struct Dft<16, INV, C> {
+  // v * (c -+ i s)
+  template <typename T> static __device__ __forceinline__ C rot(C v, T c, T s) {
+    return cmul(v, mk(c, INV ? s : -s));
+  }
+  static __device__ __forceinline__ void run(C *v) {
+    using T = typename Real<C>::type;
+    const T h = (T)FF_SQRT1_2, c = (T)FF_C16_1, s = (T)FF_S16_1;
+    C t[4][4];   // [r2][s1]
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+#pragma unroll
+      for (int r = 0; r < 4; r++) t[q][r] = v[4 * r + q];
+      Dft<4, INV, C>::run(t[q]);
+    }
+    t[1][1] = rot(t[1][1], c, s);
+    t[1][2] = cscale(cadd(t[1][2], mul_wi<INV>(t[1][2])), h);
+    t[1][3] = rot(t[1][3], s, c);
+    t[2][1] = cscale(cadd(t[2][1], mul_wi<INV>(t[2][1])), h);
+    t[2][2] = mul_wi<INV>(t[2][2]);
+    t[2][3] = cscale(csub(mul_wi<INV>(t[2][3]), t[2][3]), h);
+    t[3][1] = rot(t[3][1], s, c);
+    t[3][2] = cscale(csub(mul_wi<INV>(t[3][2]), t[3][2]), h);
+    t[3][3] = rot(t[3][3], -c, -s);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      C y[4] = {t[0][q], t[1][q], t[2][q], t[3][q]};
+      Dft<4, INV, C>::run(y);
+#pragma unroll
+      for (int r = 0; r < 4; r++) v[q + 4 * r] = y[r];
+    }
+  }
+};
+
 // ------------------------------------------------------------ radix plan
 // Radix order of a DIF transform of length n = 2^a 3^b 5^c 7^d: radix 8
 // while three factors of 2 remain, then one 4 or 2, then the 5s, the 3s and
@@ -237,10 +275,27 @@ __host__ __device__ constexpr int plan_stages(int n) {
   }
   return s > 0 ? s : 1;
 }
+// The plan of a compile-time transform: plan_radix's, or (FP32 y passes of 1024
+// points) 16 x 8 x 8, whose three stages replace the four of 8 x 8 x 8 x 2: every
+// stage reads and writes the tile once and fetches its factors from L1, which
+// bound those passes.  1024^3 FP32: the solve 13.08 -> 12.75 ms, y now 1.86 / 1.88.  The x
+// pass keeps the four (it takes the same 3040 us with 16 x 8 x 8 and 8 x 8 x 16, as
+// it is bound by the latency of its 64-byte rows), and so does FP64, whose sixteen
+// values alone fill 64 registers of 80.
+template <int N> struct CtPlan {
+  static __host__ __device__ constexpr int radix(int s) { return plan_radix(N, s); }
+  static constexpr int stages = plan_stages(N);
+};
+struct CtPlan16x8x8 {
+  static __host__ __device__ constexpr int radix(int s) { return s == 0 ? 16 : 8; }
+  static constexpr int stages = 3;
+};
+template <int N, typename C> struct YPlan { using type = CtPlan<N>; };
+template <> struct YPlan<1024, float2> { using type = CtPlan16x8x8; };
 // Span (sub-transform length) of stage s.
-__host__ __device__ constexpr int plan_span(int n, int s) {
-  int L = n;
-  for (int q = 0; q < s; q++) L /= plan_radix(n, q);
+template <int N, typename PLAN> __host__ __device__ constexpr int ct_span(int s) {
+  int L = N;
+  for (int q = 0; q < s; q++) L /= PLAN::radix(q);
   return L;
 }
 
@@ -323,6 +378,13 @@ template <typename F, typename = void> struct PairAccess : std::false_type {};
 template <typename F>
 struct PairAccess<F, std::void_t<decltype(F::kPair)>> : std::integral_constant<bool, F::kPair> {};
 
+// a, b = b, a if sw
+template <typename C> __device__ __forceinline__ void exchange(int sw, C &a, C &b) {
+  const C t = a;
+  a = sw ? b : a;
+  b = sw ? t : b;
+}
+
 // A point-major FP32 stage with two adjacent columns per item: the pair moves
 // as one 16-byte shared-memory access, and the row group's twiddles are loaded
 // (or generated) once for both columns.  Same arithmetic per value as stage().
@@ -339,10 +401,13 @@ __device__ __forceinline__ void stage_pairs(int n_rt, int L_rt, const AxisDev<fl
   // the last DIF stage of radix 2 on 64-byte rows: odd items read their rows
   // swapped (see stage())
   constexpr bool kSwap = R == 2 && !DIT && W * sizeof(float2) == 64;
+  // other even radices: they exchange the two rows' values after the loads
+  // (1024^3 FP32 y 1889 / 1902 -> 1861 / 1889 us)
+  constexpr bool kExchange = R > 2 && R % 2 == 0 && !DIT && W * sizeof(float2) == 64 && LC == R;
   auto body = [&](int it) {
     const int c = 2 * (it % WP);
     const int b = it / WP;
-    const int sw = kSwap && m == 1 ? b & 1 : 0;
+    const int sw = (kSwap && m == 1) || kExchange ? b & 1 : 0;
     int blk, j;
     if (NC) {
       blk = b / m;
@@ -379,6 +444,13 @@ __device__ __forceinline__ void stage_pairs(int n_rt, int L_rt, const AxisDev<fl
       u[r] = make_float2(q.x, q.y);
       v[r] = make_float2(q.z, q.w);
     }
+    if constexpr (kExchange) {
+#pragma unroll
+      for (int r = 0; r < R; r += 2) {
+        exchange(sw, u[r], u[r + 1]);
+        exchange(sw, v[r], v[r + 1]);
+      }
+    }
     auto apply = [&](float2 *x) {
 #pragma unroll
       for (int r = 1; r < R; r++) x[r] = cmul(x[r], w[r - 1]);
@@ -397,7 +469,7 @@ __device__ __forceinline__ void stage_pairs(int n_rt, int L_rt, const AxisDev<fl
         apply(u);
         apply(v);
       }
-      if (sw) {
+      if (kSwap && sw) {
         u[R - 1] = make_float2(-u[R - 1].x, -u[R - 1].y);
         v[R - 1] = make_float2(-v[R - 1].x, -v[R - 1].y);
       }
@@ -420,7 +492,8 @@ template <int R, bool INV, bool DIT, Map MAP, int W, int NT, int NC, int LC, boo
 __device__ __forceinline__ void stage(int n_rt, int L_rt, const AxisDev<C> &ax, LD &ld, ST &st, int ncols) {
   // compile-time plans only: a runtime plan instantiates every radix, and the
   // paired registers of all of them spilled
-  if constexpr (NC > 0 && std::is_same<C, float2>::value && MAP == Map::ColFast && W % 2 == 0 &&
+  // (radix 16: one column per item, a pair's 32 values do not fit the registers)
+  if constexpr (NC > 0 && std::is_same<C, float2>::value && MAP == Map::ColFast && W % 2 == 0 && R < 16 &&
                 PairAccess<LD>::value && PairAccess<ST>::value) {
     stage_pairs<R, INV, DIT, W, NT, NC, LC, TWREC, TWMUL>(n_rt, L_rt, ax, ld, st);
     return;
@@ -457,8 +530,8 @@ __device__ __forceinline__ void stage(int n_rt, int L_rt, const AxisDev<C> &ax, 
     // Stage with twiddles: the factors are fetched before the data loads and
     // applied without a branch (j = 0 reads exp(0) = 1), so their latency
     // overlaps the data loads.  Not for FP64 line-major tiles, where the
-    // extra live registers spill.
-    constexpr bool kPrefetch = !(MAP == Map::PosFast && sizeof(C) == 16);
+    // extra live registers spill, and not for radix 16.
+    constexpr bool kPrefetch = !(MAP == Map::PosFast && sizeof(C) == 16) && R < 16;
     // runtime plans take the same path in every stage that has twiddles
     // (span above the radix); the branch is uniform across the block
     bool pf = false;
@@ -520,7 +593,7 @@ __device__ __forceinline__ void stage(int n_rt, int L_rt, const AxisDev<C> &ax, 
   };
   if constexpr (NC > 0 && NT > 0 && MAP == Map::ColFast && (W * (NC / R)) % NT == 0) {
     constexpr int ITER = W * (NC / R) / NT;
-#pragma unroll
+#pragma unroll(R < 16 ? ITER : 1)
     for (int q = 0; q < ITER; q++) body((int)threadIdx.x + q * NT);
   } else {
     const int items = ncols * nb;
@@ -640,11 +713,11 @@ template <int N> __device__ __forceinline__ int group_of_base(int k0) {
 
 // Digit reversal of a compile-time plan: the frequency held at DIF output
 // position pos (the host builds the same table for runtime plans).
-template <int N> __device__ __forceinline__ int rev_ct(int pos) {
+template <int N, typename PLAN = CtPlan<N>> __device__ __forceinline__ int rev_ct(int pos) {
   int k = 0, kmul = 1, span = N;
 #pragma unroll
-  for (int s = 0; s < plan_stages(N); s++) {
-    const int r = plan_radix(N, s);
+  for (int s = 0; s < PLAN::stages; s++) {
+    const int r = PLAN::radix(s);
     span /= r;
     const int m = pos / span;
     pos -= m * span;
@@ -667,8 +740,8 @@ template <int RC = 0, int NRC = 0> struct RevLast {
   }
 };
 
-template <int N> struct RevCT {
-  __device__ __forceinline__ int operator()(int pos) const { return rev_ct<N>(pos); }
+template <int N, typename PLAN = CtPlan<N>> struct RevCT {
+  __device__ __forceinline__ int operator()(int pos) const { return rev_ct<N, PLAN>(pos); }
 };
 
 // Line-major tile written at the natural (frequency) index of a DIF output
@@ -720,18 +793,18 @@ __device__ __forceinline__ void dit_rt(const AxisDev<C> &ax, int s_begin, MID &m
 // TWREC0: recurrence twiddles in stage 0; TWALL: in every stage.
 // TWMUL: the axis table is TWMUL times longer than N (N is a sub-transform).
 template <int N, int SEND, int s, bool INV, Map MAP, int W, int NT, bool TWREC0, bool TWALL, int TWMUL = 1,
-          typename C, typename LD0, typename MID, typename STL>
+          typename PLAN = CtPlan<N>, typename C, typename LD0, typename MID, typename STL>
 __device__ __forceinline__ void dif_ct(const AxisDev<C> &ax, LD0 &ld0, MID &mid, STL &stl, int ncols) {
   if constexpr (s < SEND) {
-    constexpr int R = plan_radix(N, s);
-    constexpr int L = plan_span(N, s);
+    constexpr int R = PLAN::radix(s);
+    constexpr int L = ct_span<N, PLAN>(s);
     constexpr bool TWR = TWALL || (TWREC0 && s == 0);
     if constexpr (s == 0 && SEND == 1) stage<R, INV, false, MAP, W, NT, N, L, TWR, TWMUL>(N, L, ax, ld0, stl, ncols);
     else if constexpr (s == 0) stage<R, INV, false, MAP, W, NT, N, L, TWR, TWMUL>(N, L, ax, ld0, mid, ncols);
     else if constexpr (s == SEND - 1) stage<R, INV, false, MAP, W, NT, N, L, TWR, TWMUL>(N, L, ax, mid, stl, ncols);
     else stage<R, INV, false, MAP, W, NT, N, L, TWR, TWMUL>(N, L, ax, mid, mid, ncols);
     __syncthreads();
-    dif_ct<N, SEND, s + 1, INV, MAP, W, NT, TWREC0, TWALL, TWMUL>(ax, ld0, mid, stl, ncols);
+    dif_ct<N, SEND, s + 1, INV, MAP, W, NT, TWREC0, TWALL, TWMUL, PLAN>(ax, ld0, mid, stl, ncols);
   }
 }
 
@@ -741,7 +814,7 @@ template <int N, int s, bool INV, Map MAP, int W, int NT, bool TWALL, int TWMUL 
 __device__ __forceinline__ void dit_ct(const AxisDev<C> &ax, MID &mid, STL &stl, int ncols) {
   if constexpr (s >= 0) {
     constexpr int R = plan_radix(N, s);
-    constexpr int L = plan_span(N, s);
+    constexpr int L = ct_span<N, CtPlan<N>>(s);
     if constexpr (s == 0) stage<R, INV, true, MAP, W, NT, N, L, TWALL, TWMUL>(N, L, ax, mid, stl, ncols);
     else stage<R, INV, true, MAP, W, NT, N, L, TWALL, TWMUL>(N, L, ax, mid, mid, ncols);
     __syncthreads();
@@ -750,10 +823,10 @@ __device__ __forceinline__ void dit_ct(const AxisDev<C> &ax, MID &mid, STL &stl,
 }
 
 // Full DIF transform (all stages) with a compile-time (N > 0) or runtime plan.
-template <int N, bool INV, Map MAP, int W, int NT, bool TWREC0, bool TWALL, typename C, typename LD0, typename MID,
-          typename STL>
+template <int N, bool INV, Map MAP, int W, int NT, bool TWREC0, bool TWALL, typename PLAN = CtPlan<N>, typename C,
+          typename LD0, typename MID, typename STL>
 __device__ __forceinline__ void dif_all(const AxisDev<C> &ax, LD0 &ld0, MID &mid, STL &stl, int ncols) {
-  if constexpr (N > 0) dif_ct<N, plan_stages(N), 0, INV, MAP, W, NT, TWREC0, TWALL>(ax, ld0, mid, stl, ncols);
+  if constexpr (N > 0) dif_ct<N, PLAN::stages, 0, INV, MAP, W, NT, TWREC0, TWALL, 1, PLAN>(ax, ld0, mid, stl, ncols);
   else dif_rt<INV, MAP, W, NT, TWREC0, TWALL>(ax, ax.nstages, ld0, mid, stl, ncols);
 }
 

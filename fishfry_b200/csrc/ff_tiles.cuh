@@ -25,11 +25,12 @@ constexpr int kZThreads = 256;
 
 // Frequency of a last-stage DIF position: arithmetic for compile-time plans,
 // one table load per radix group otherwise.
-template <int N> struct RevLastOf { using type = RevCT<N>; };
-template <> struct RevLastOf<0> { using type = RevLast<0, 0>; };
-template <int N, typename C> __device__ __forceinline__ typename RevLastOf<N>::type rev_last(const AxisDev<C> &ax) {
+template <int N, typename PLAN = CtPlan<N>> struct RevLastOf { using type = RevCT<N, PLAN>; };
+template <typename PLAN> struct RevLastOf<0, PLAN> { using type = RevLast<0, 0>; };
+template <int N, typename PLAN = CtPlan<N>, typename C>
+__device__ __forceinline__ typename RevLastOf<N, PLAN>::type rev_last(const AxisDev<C> &ax) {
   if constexpr (N > 0) {
-    return RevCT<N>{};
+    return RevCT<N, PLAN>{};
   } else {
     const int R = ax.radix[ax.nstages - 1];
     return RevLast<0, 0>{ax.rev, R, ax.n / R};
@@ -615,10 +616,11 @@ __device__ __forceinline__ void y_tile_rows(LD0 &ld0, const RowAt &row_at, const
   using C = typename Cplx<T>::type;
   const AxisDev<C> &ax = a.ax[1];
   const int ncol = min(W, a.nh - kt * W);
-  const auto rl = rev_last<N>(ax);
+  using Plan = typename YPlan<N, C>::type;
+  const auto rl = rev_last<N, Plan>(ax);
   PointTile<W, C> tile{sm};
   RowStore<C, RowAt, std::remove_const_t<decltype(rl)>> gst{row_at, rl, ncol};
-  dif_all<N, INV, Map::ColFast, W, kZThreads, false, (sizeof(T) == 8)>(ax, ld0, tile, gst, W);
+  dif_all<N, INV, Map::ColFast, W, kZThreads, false, (sizeof(T) == 8), Plan>(ax, ld0, tile, gst, W);
 }
 
 // y transform of one tile of plane o, stored into the spectrum dst at the
