@@ -349,7 +349,7 @@ __device__ __forceinline__ bool batch_tile(const GridHead<T> &g, const KindDesc 
         switch (a.nk) {
 #define FF_CASE(NN) \
   case NN: {                                                                              \
-    const bool ok = z_fwd_tile<T, NN, true, true, true, kBatchZThreads>(g.density, spec, a, zW, P, line0, nlines, sm, io); \
+    const bool ok = z_fwd_tile<T, NN, true, kBatchZThreads>(g.density, spec, a, zW, P, line0, nlines, sm, io); \
     parity ^= 1u;                                                                         \
     return ok;                                                                            \
   }
@@ -366,7 +366,7 @@ __device__ __forceinline__ bool batch_tile(const GridHead<T> &g, const KindDesc 
         switch (a.nk) {
 #define FF_CASE(NN)                                                                       \
   case NN: {                                                                              \
-    const bool ok = z_inv_tile<T, NN, true, true, kBatchZThreads>(spec, g.potential, a, zW, P, line0, nlines, sm, io); \
+    const bool ok = z_inv_tile<T, NN, true, kBatchZThreads>(spec, g.potential, a, zW, P, line0, nlines, sm, io); \
     parity ^= 1u;                                                                         \
     return ok;                                                                            \
   }

@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kZPassThreads, 6) k_zfwd(const T *__restrict__
       l2_prefetch(f + fl * a.nk, (uint32_t)(min((long)(2 * W), nlines - fl) * a.nk * sizeof(T)));
   }
   const ZTileIO io{&mbar, 0, a.status, a.wait_iters};
-  z_fwd_tile<T, N, true, true, true, kZPassThreads>(f, spec, a, W, P, (long)blockIdx.x * (2 * W), nlines,
+  z_fwd_tile<T, N, true, kZPassThreads>(f, spec, a, W, P, (long)blockIdx.x * (2 * W), nlines,
                                reinterpret_cast<typename Cplx<T>::type *>(align128(smraw)), io);
 }
 
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(kZPassThreads, 6) k_zinv(const typename Cplx<T
                   (uint32_t)(min((long)(2 * W), nlines - fl) * a.nhp * sizeof(typename Cplx<T>::type)));
   }
   const ZTileIO io{&mbar, 0, a.status, a.wait_iters};
-  z_inv_tile<T, N, true, true, kZPassThreads>(spec, out, a, W, P, (long)blockIdx.x * (2 * W), nlines,
+  z_inv_tile<T, N, true, kZPassThreads>(spec, out, a, W, P, (long)blockIdx.x * (2 * W), nlines,
                          reinterpret_cast<typename Cplx<T>::type *>(align128(smraw)), io);
 }
 

@@ -52,11 +52,11 @@ __device__ __forceinline__ typename RevLastOf<N, PLAN>::type rev_last(const Axis
 // registers.
 // A holds max(W*P, 2W*nhp) complex values, B holds W*P (+ 128 bytes slack).
 //
-// LASTFUSE (single-grid passes, compile-time plans with a radix-8 prefix):
-// the last stage is fused with the split (forward) or with the scatter of the
-// two real lines (inverse), so the stages' output never goes through shared
-// memory in natural order.  Forward: stages in A (LineTileZ), the last stage
-// writes the staged spectrum rows into B, which then also holds
+// With TMAIO and a compile-time plan of a radix-8 prefix, the last stage is
+// fused with the split (forward) or with the scatter of the two real lines
+// (inverse), so the stages' output never goes through shared memory in natural
+// order.  Forward: stages in A (LineTileZ), the last stage writes the staged
+// spectrum rows into B, which then also holds
 // max(W*P, 2W*nhp) values.  Inverse: stages in B (LineTileZ), the last stage
 // writes the real lines into A.
 struct ZTileIO {
@@ -257,7 +257,7 @@ __device__ __forceinline__ void z_inv_last_stage(const LineTileZ<C> &t, typename
 // order into B; the split A[k] = (Z[k] + conj Z[n-k]) / 2,
 // B[k] = (Z[k] - conj Z[n-k]) / (2i) goes out with consecutive threads on
 // consecutive k.
-template <typename T, int N, bool TMAIO, bool TMA_OUT = TMAIO, bool LASTFUSE = false, int NT = kZThreads>
+template <typename T, int N, bool TMAIO, int NT = kZThreads>
 __device__ __forceinline__ bool z_fwd_tile(const T *__restrict__ f, typename Cplx<T>::type *spec, const PassArgs<T> &a,
                                            int W, int P, long line0, long lend, typename Cplx<T>::type *sm,
                                            const ZTileIO &io) {
@@ -283,7 +283,7 @@ __device__ __forceinline__ bool z_fwd_tile(const T *__restrict__ f, typename Cpl
       const int la = 2 * c;
       return mk(la < nl ? raw[la * nk + pos] : (T)0, la + 1 < nl ? raw[(la + 1) * nk + pos] : (T)0);
     };
-    if constexpr (LASTFUSE && TMA_OUT && N > 0 && radix8_prefix(N) && z_split_fused(N, sizeof(C))) {
+    if constexpr (N > 0 && radix8_prefix(N) && z_split_fused(N, sizeof(C))) {
       // stages in A, the fused last stage stages the spectrum rows in B
       LineTileZ<C> tAz{A, P};
       dif_ct<N, plan_stages(N) - 1, 0, false, Map::PosFast, 1, NT, true, true>(ax, ld0, tAz, tAz, W);
@@ -320,32 +320,16 @@ __device__ __forceinline__ bool z_fwd_tile(const T *__restrict__ f, typename Cpl
     };
     dif_all<N, false, Map::PosFast, 1, NT, true, true>(ax, ldg, tA, tBrev, W);
     const T h = (T)0.5;
-    if constexpr (TMA_OUT) {
-      // staged rows [line][kh] (pitch nhp) in A, then one copy out
-      for (int it = threadIdx.x; it < W * nha; it += NT) {
-        const int k = it % nha;
-        const int c = it / nha;
-        if (k >= nh) continue;
-        const C z = tB(k, c);
-        const C w = tB(k == 0 ? 0 : nk - k, c);
-        A[(2 * c) * a.nhp + k] = mk(h * (z.x + w.x), h * (z.y - w.y));
-        A[(2 * c + 1) * a.nhp + k] = mk(h * (z.y + w.y), h * (w.x - z.x));
-      }
-      fence_proxy_async_smem();
-      __syncthreads();
-      bulk_out(spec + line0 * a.nhp, A, (size_t)nl * a.nhp);
-    } else {
-      for (int it = threadIdx.x; it < W * nha; it += NT) {
-        const int k = it % nha;
-        const int c = it / nha;
-        if (k >= nh) continue;
-        const long la = line0 + 2 * c;
-        if (la >= lend) continue;
-        const C z = tB(k, c);
-        const C w = tB(k == 0 ? 0 : nk - k, c);
-        spec[la * a.nhp + k] = mk(h * (z.x + w.x), h * (z.y - w.y));
-        if (la + 1 < lend) spec[(la + 1) * a.nhp + k] = mk(h * (z.y + w.y), h * (w.x - z.x));
-      }
+    for (int it = threadIdx.x; it < W * nha; it += NT) {
+      const int k = it % nha;
+      const int c = it / nha;
+      if (k >= nh) continue;
+      const long la = line0 + 2 * c;
+      if (la >= lend) continue;
+      const C z = tB(k, c);
+      const C w = tB(k == 0 ? 0 : nk - k, c);
+      spec[la * a.nhp + k] = mk(h * (z.x + w.x), h * (z.y - w.y));
+      if (la + 1 < lend) spec[(la + 1) * a.nhp + k] = mk(h * (z.y + w.y), h * (w.x - z.x));
     }
     return true;
   }
@@ -355,7 +339,7 @@ __device__ __forceinline__ bool z_fwd_tile(const T *__restrict__ f, typename Cpl
 // Hermitian extension in natural order in B (the imaginary parts of the zero
 // and Nyquist terms are dropped, as a C2R transform does), inverse DIF into
 // natural order in B, real and imaginary parts out to the two lines.
-template <typename T, int N, bool TMAIO, bool LASTFUSE = false, int NT = kZThreads>
+template <typename T, int N, bool TMAIO, int NT = kZThreads>
 __device__ __forceinline__ bool z_inv_tile(const typename Cplx<T>::type *spec, T *__restrict__ out,
                                            const PassArgs<T> &a, int W, int P, long line0, long lend,
                                            typename Cplx<T>::type *sm, const ZTileIO &io) {
@@ -399,7 +383,7 @@ __device__ __forceinline__ bool z_inv_tile(const typename Cplx<T>::type *spec, T
       if (k == 0 || 2 * k == nk) return mk(sa.x, sb.x);
       return lo ? mk(sa.x - sb.y, sa.y + sb.x) : mk(sa.x + sb.y, sb.x - sa.y);
     };
-    if constexpr (LASTFUSE && N > 0 && radix8_prefix(N)) {
+    if constexpr (N > 0 && radix8_prefix(N)) {
       // stages in B, the fused last stage writes the real lines into A
       LineTileZ<C> tBz{B, P};
       dif_ct<N, plan_stages(N) - 1, 0, true, Map::PosFast, 1, NT, true, true>(ax, ldh, tBz, tBz, W);
