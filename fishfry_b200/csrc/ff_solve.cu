@@ -872,6 +872,11 @@ int ff_plan_create(const int n[3], const double lo[3], const double hi[3], int p
       return set_error(FF_ERR_UNSUPPORTED, "ff_plan_create: too many stages");
     }
     rev[d] = plan_digit_reversal(L, radix[d]);
+    // FP64 compile-time tables start on 16 KB: every SM reads their few lines all the
+    // time, and how those spread over the L2 depends on the address (512-point y
+    // tables 8, 12, 16, 20, 24, 32 KB into the plan: 363, 369, 346, 373, 367, 373 us for
+    // the forward y pass of 512^3, and 354 at 16 KB against 373-389 in 1024x512x256)
+    if (precision == FF_FP64 && special_n(n[d])) off = (off + 16383) & ~size_t(16383);
     o_tw[d] = take(L * csz);
     o_tw64[d] = precision == FF_FP64 ? o_tw[d] : take(L * sizeof(double2));
   }
