@@ -631,7 +631,7 @@ def batch_dims(seed=2024, count=256, choices=(32, 48, 64, 80, 96, 128)):
 
 def batch_measure(steps, warmup, seed, tune=True):
     """256 grids with dims iid from {32, 48, 64, 80, 96, 128}: batched solves
-    (five persistent launches, graph replay, tuned tiles) in FP64 and FP32
+    (five launches, graph replay, tuned tiles) in FP64 and FP32
     against a loop of single-grid FP64 solves of the same grids; errors
     against those plain FP64 solves, computed on the device."""
     import torch
@@ -739,7 +739,7 @@ def run_batch(args):
         "value": r["fp32_batch"]["solves_per_s"], "unit": "solves/s", "n_gpus": 1, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": r["fp32_batch"]["ms"], "higher_is_better": True, "dtype": "f32",
         "data": "synthetic: " + r["data"], "config": {
-            "workload": "256 grids, dims seed 2024, five persistent launches per solve (CUDA graph), %s tiles" %
+            "workload": "256 grids, dims seed 2024, five launches per solve (CUDA graph), %s tiles" %
                         r["tiles"], "points_per_batch": r["points_per_batch"]},
     }
     line.update({k: v for k, v in r.items() if k not in ("data",)})
