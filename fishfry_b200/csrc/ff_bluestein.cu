@@ -468,8 +468,8 @@ int rader_root(int n) {
 }
 
 // The cheapest 2^a 3^b 5^c 7^d length from 2n - 1 to a third more, by the cost
-// of its stages (a length of fewer, better radices is worth some padding: 251
-// points go through 512 = 8 x 8 x 8, not 504 = 8 x 7 x 9); above 1500 points the
+// of its stages (a length of fewer, better radices is worth some padding: from 501
+// on 512 = 8 x 8 x 8, not 504 = 9 x 8 x 7); above 1500 points the
 // smallest, whose tile has to fit.
 int bs_padded_length(int n) {
   const int lo = std::max(1, 2 * n - 1), hi = n > 1500 ? lo : lo + lo / 3;
