@@ -485,7 +485,7 @@ __global__ void __launch_bounds__((KIND == 0 || KIND == 4) ? kBatchZThreads : kZ
         const long l1 = min(l0 + 2 * zW, nlines);
         const size_t b0 = (l0 * row) & ~size_t(15);
         const size_t b1 = min((l1 * row + 15) & ~size_t(15), cap & ~size_t(15));
-        if (b1 > b0) l2_prefetch(reinterpret_cast<const char *>(G->h.density) + b0, (uint32_t)(b1 - b0));
+        l2_prefetch(reinterpret_cast<const char *>(G->h.density) + b0, (uint32_t)(b1 - b0));
       }
     }
   }

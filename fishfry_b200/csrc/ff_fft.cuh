@@ -922,10 +922,12 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 // shared memory (the buffer may then be reused or released).
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 
-// L2 prefetch hint of a contiguous range (16-byte aligned, size a multiple of
-// 16).  No data reaches shared memory and no completion is tracked.
+// L2 prefetch hint of the whole 16-byte units of a contiguous range that starts
+// on 16 bytes; a range with none (one line of fewer than 16 bytes) is not hinted.
+// No data reaches shared memory and no completion is tracked.
 __device__ __forceinline__ void l2_prefetch(const void *src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+  bytes &= ~15u;
+  if (bytes) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 
 // Element copies from global to shared memory that complete asynchronously

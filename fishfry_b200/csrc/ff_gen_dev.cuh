@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(256, 3)
   }
   if (threadIdx.x == blockDim.x - 1 && a.l2_ahead > 0) {
     const long fl = b.line0 + (long)a.l2_ahead * b.lines;
-    if (fl < nlines) l2_prefetch(src + fl * rin, (uint32_t)(min((long)b.lines, nlines - fl) * rin) & ~15u);
+    if (fl < nlines) l2_prefetch(src + fl * rin, (uint32_t)(min((long)b.lines, nlines - fl) * rin));
   }
   __syncthreads();
   if (!z_wait(&mbar, a.status, a.wait_iters)) return;
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(256, 3)
     // the lines of the block one resident wave ahead into L2
     const long fl = ((long)blockIdx.x + a.l2_ahead) * lines;
     if (fl < nlines)
-      l2_prefetch(f + fl * nk, (uint32_t)((size_t)min((long)lines, nlines - fl) * nk * sizeof(T)) & ~15u);
+      l2_prefetch(f + fl * nk, (uint32_t)((size_t)min((long)lines, nlines - fl) * nk * sizeof(T)));
   }
   if (!z_wait(&mbar, a.status, a.wait_iters)) return;
   if (nl < lines) {
