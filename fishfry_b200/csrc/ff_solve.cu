@@ -748,6 +748,10 @@ int plan_launch_z(const ff_plan *p, bool inverse, void *in, void *out, cudaStrea
                                  : launch_z<float>(p, inverse, in, out, st);
 }
 
+// The first passes of a solve end on a kernel that has called pdl_start; this one,
+// launched plainly after it, makes what follows on the stream follow the pass.
+__global__ void k_end_of_call() {}
+
 static int plan_phases(const ff_plan *p) { return p->fused ? 3 : 5; }
 
 // Reads and clears the device status word; FF_ERR_TIMEOUT if a bounded wait
@@ -1039,8 +1043,12 @@ int ff_solve_passes(const ff_plan *p, size_t bytes, void *density, void *potenti
   if (((uintptr_t)density | (uintptr_t)potential) & 15)
     return set_error(FF_ERR_INVALID, "ff_solve_passes: buffers must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  return p->precision == FF_FP64 ? launch_solve<double>(p, density, potential, st, false, passes)
-                                 : launch_solve<float>(p, density, potential, st, false, passes);
+  const int rc = p->precision == FF_FP64 ? launch_solve<double>(p, density, potential, st, false, passes)
+                                         : launch_solve<float>(p, density, potential, st, false, passes);
+  if (rc != FF_OK || passes == 5) return rc;
+  k_end_of_call<<<1, 1, 0, st>>>();
+  FF_CUDA(cudaGetLastError());
+  return FF_OK;
 }
 
 int ff_plan_check(const ff_plan *p, void *stream) {
