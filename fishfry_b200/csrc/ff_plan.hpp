@@ -52,7 +52,7 @@ struct ff_plan {
   size_t zsmem;
   unsigned ztiles;
   bool chained;        // passes as programmatic dependents of one another (ff_launch.hpp)
-  int l2_ahead;        // forward z pass: L2 prefetch distance in blocks (0: off)
+  int l2_ahead;        // z passes: L2 prefetch distance in blocks (0: off)
   int wait_iters;      // bounded device waits: iteration limit of the first wait (0: built-in)
   int dep_extra;       // fused passes: added to every dependency wait's target (test hook, 0)
   ff::StridedCfg ycfg, xcfg;
@@ -96,11 +96,12 @@ template <typename T> PassArgs<T> pass_args(const ff_plan *p) {
 }
 
 // The generic (or Bluestein) passes' arguments of axis d with the plan's
-// current wait limit.
+// L2 prefetch distance (z passes) and current wait limit.
 template <typename T> GenPass<typename Cplx<T>::type> gen_pass(const ff_plan *p, int d) {
   GenPass<typename Cplx<T>::type> a;
   if constexpr (sizeof(T) == 8) a = p->gpd[d];
   else a = p->gpf[d];
+  a.l2_ahead = p->l2_ahead;
   a.wait_iters = p->wait_iters;
   return a;
 }
@@ -121,6 +122,9 @@ int encode_spectrum_map(void *base, int ni, int nj, int nh, int nhp, size_t esz,
 // Raises fn's dynamic shared-memory limit to what is left beside its static
 // shared memory; returns that limit in *avail (may be NULL).
 int allow_dyn_smem_fn(const void *fn, size_t *avail);
+
+// The L2 prefetch distance of a plan's z passes in blocks, as their launches take it.
+int plan_l2_ahead(const ff_plan *p);
 
 // The z forward (inverse = false: real field `in` -> half spectrum `out`) or z
 // inverse (spectrum `in` -> real field `out`) pass of plan p on stream st,

@@ -539,9 +539,7 @@ template <typename T> static int configure(ff_plan *p) {
       g.invN = 1.0 / (double(ni) * double(nj) * double(nk));
       g.status = p->status;
       g.wait_iters = 0;
-      // the resident blocks' successors (as the compile-time z passes do)
-      const int per_sm = std::max(1, std::min((int)(kMaxDynSmem / (sh.smem + 1024)), 768 / sh.threads));
-      g.l2_ahead = per_sm * p->num_sms;
+      g.l2_ahead = 0;   // the plan's, at the launch (gen_pass)
     };
     if constexpr (sizeof(T) == 8) {
       if (p->gen[d]) fill(p->gpd[d]);
@@ -588,13 +586,21 @@ template <typename T> static int configure(ff_plan *p) {
     const int per_plane = fc.prod_pp + fc.cons_pp;
     fc.lag = std::min(ni, std::max(2, (3 * fc.grid + 2 * per_plane - 1) / (2 * per_plane)));
   }
-  // The z passes run one tile per block, six blocks per SM, each waiting for
-  // its inbound line block.  Block b hints block b + l2_ahead's lines
-  // (forward) or spectrum rows (inverse) into L2, so that read is under way
-  // while the resident blocks compute and the later bulk copy finds them in
-  // L2.  (The same hint on the strided passes' tensor tiles slowed them.)
+  // The z passes run one tile per block, each waiting for its inbound line
+  // block.  Block b hints block b + l2_ahead's lines (forward) or spectrum rows
+  // (inverse) into L2, so that read is under way while the resident blocks compute
+  // and the later bulk copy finds them in L2: one wave ahead, six blocks per SM for
+  // the compile-time kernels and what the tile lets for the generic ones, or as
+  // the environment says (FF_L2_AHEAD, 0: no hints).  (The same hint on the
+  // strided passes' tensor tiles slowed them; the convolutions of Bluestein axes,
+  // bound by their stages, take none.)
+  int per_sm = 6;
+  if (p->gen[2]) {
+    const GenShape &sh = p->gshape[2];
+    per_sm = std::max(1, std::min((int)(kMaxDynSmem / (sh.smem + 1024)), 768 / sh.threads));
+  }
   const char *ahead = getenv("FF_L2_AHEAD");
-  p->l2_ahead = ahead ? std::max(0, atoi(ahead)) : 6 * p->num_sms;
+  p->l2_ahead = ahead ? std::max(0, atoi(ahead)) : per_sm * p->num_sms;
   return FF_OK;
 }
 
@@ -742,6 +748,8 @@ int allow_dyn_smem_fn(const void *fn, size_t *avail) {
   if (avail) *avail = lim;
   return FF_OK;
 }
+
+int plan_l2_ahead(const ff_plan *p) { return p->l2_ahead; }
 
 int plan_launch_z(const ff_plan *p, bool inverse, void *in, void *out, cudaStream_t st) {
   return p->precision == FF_FP64 ? launch_z<double>(p, inverse, in, out, st)
