@@ -10,6 +10,7 @@
 #include <cstdint>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "ff_status.hpp"
 
@@ -23,8 +24,20 @@ struct FieldArgs {
   int ni, nj, nk;
   double xlo, ylo, zlo, dx, dy, dz;
   int nmodes;
+  int split;   // an amplitude is not finite: weights stay apart from the cosines (kSplitModes)
   ff_mode modes[kMaxModes];
 };
+
+// What a kernel is built for: no modes, modes whose weights its tables hold, or
+// modes with a weight that is not finite (cos A cos B - sin A sin B would be inf -
+// inf), which multiplies the point's cosine as the formula has it.
+enum : int { kNoModes = 0, kModes = 1, kSplitModes = 2 };
+
+// Weight of a mode in f or in phi; the zero mode counts as absent.
+__device__ __forceinline__ int mode_k2(const ff_mode &m) { return m.kx * m.kx + m.ky * m.ky + m.kz * m.kz; }
+__device__ __forceinline__ double mode_weight(const ff_mode &m, bool solution) {
+  return solution ? -m.a / (double)mode_k2(m) : m.a;
+}
 
 // phi factors and their second derivatives along one axis, FishFry.hpp:22-41
 // and :71-86: (factor, second derivative) at one coordinate.
@@ -72,7 +85,7 @@ struct FieldTiles {
 
 // Values of the tile's 16 points of this thread: f (solution = false) or phi,
 // summed as the point-by-point formulas are (FishFry.hpp:44, :87).
-template <bool MODES>
+template <int MODES>
 __device__ __forceinline__ void tile_values(const FieldArgs &a, const double2 *sm, int warp, int lane, bool solution,
                                             double v[kTileWarpLines][2]) {
   const double2 *zf = sm, *lx = sm + kTileK, *ly = lx + kTileLines;
@@ -85,10 +98,20 @@ __device__ __forceinline__ void tile_values(const FieldArgs &a, const double2 *s
     for (int q = 0; q < 2; q++)
       v[l][q] = solution ? x.x * y.x * z[q].x : x.x * y.x * z[q].y + x.x * y.y * z[q].x + x.y * y.x * z[q].x;
   }
-  if constexpr (!MODES) return;
+  if constexpr (MODES == kNoModes) return;
   double s[kTileWarpLines][2] = {};
   for (int m = 0; m < a.nmodes; m++) {
     const double2 b0 = zm[m * kTileK + lane], b1 = zm[m * kTileK + lane + 32];
+    if constexpr (MODES == kSplitModes) {
+      if (mode_k2(a.modes[m]) == 0) continue;
+      const double w = mode_weight(a.modes[m], solution);
+      for (int l = 0; l < kTileWarpLines; l++) {
+        const double2 c = lm[m * kTileLines + warp * kTileWarpLines + l];
+        s[l][0] = fma(w, c.x * b0.x - c.y * b0.y, s[l][0]);
+        s[l][1] = fma(w, c.x * b1.x - c.y * b1.y, s[l][1]);
+      }
+      continue;
+    }
 #pragma unroll
     for (int l = 0; l < kTileWarpLines; l++) {
       const double2 w = lm[m * kTileLines + warp * kTileWarpLines + l];   // weight times (cos A, sin A)
@@ -134,19 +157,20 @@ __device__ __forceinline__ void line_tables(const FieldArgs &a, double2 *sm, lon
     } else if (q < 2 * kTileLines) {
       ly[q - kTileLines] = factor_y(y);
     } else {
-      // weight a (f) or -a / |k|^2 (phi); the zero mode counts as absent
-      const int m = q / kTileLines - 2;
-      const ff_mode &md = a.modes[m];
-      const int k2 = md.kx * md.kx + md.ky * md.ky + md.kz * md.kz;
-      const double w = k2 == 0 ? 0.0 : solution ? -md.a / (double)k2 : md.a;
-      double s, c;
-      sincos((double)md.kx * x + (double)md.ky * y + md.theta, &s, &c);
-      lm[q - 2 * kTileLines] = make_double2(w * c, w * s);
+      // weight a (f) or -a / |k|^2 (phi) times the line's cosine and sine
+      const ff_mode &md = a.modes[q / kTileLines - 2];
+      double2 v = make_double2(0.0, 0.0);
+      if (mode_k2(md) != 0) {
+        const double w = a.split ? 1.0 : mode_weight(md, solution);
+        sincos((double)md.kx * x + (double)md.ky * y + md.theta, &v.y, &v.x);
+        v = make_double2(w * v.x, w * v.y);
+      }
+      lm[q - 2 * kTileLines] = v;
     }
   }
 }
 
-template <typename T, bool MODES>
+template <typename T, int MODES>
 __global__ void __launch_bounds__(kSumThreads, MODES ? 2 : 4) k_init(const FieldArgs a, const FieldTiles t, T *__restrict__ f) {
   extern __shared__ double2 smf[];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -179,7 +203,7 @@ __global__ void __launch_bounds__(kSumThreads, MODES ? 2 : 4) k_init(const Field
 // tree; the grid is a function of the dimensions alone, so the sums are
 // reproducible.  NaN propagates through the max, as the reference's integer
 // atomicMax on the bit pattern does.
-template <typename T, bool MODES>
+template <typename T, int MODES>
 __global__ void __launch_bounds__(kSumThreads, MODES ? 2 : 3) k_diff(const FieldArgs a, const FieldTiles t, const T *__restrict__ phi,
                                                       double *__restrict__ partial) {
   __shared__ double s1[kSumThreads], s2[kSumThreads], sm[kSumThreads];
@@ -291,7 +315,10 @@ static int field_args(const int n[3], const double xlo[3], const double dx[3], i
   a.dy = dx[1];
   a.dz = dx[2];
   a.nmodes = nmodes;
-  for (int m = 0; m < nmodes; m++) a.modes[m] = modes[m];
+  for (int m = 0; m < nmodes; m++) {
+    a.modes[m] = modes[m];
+    if (!std::isfinite(modes[m].a)) a.split = 1;
+  }
   return FF_OK;
 }
 
@@ -323,6 +350,13 @@ template <typename F> static int allow_tables(F fn, size_t smem) {
   return FF_OK;
 }
 
+// Calls f with the kernels' form as a constant.
+template <typename F> static int with_modes(const FieldArgs &a, F &&f) {
+  if (a.nmodes == 0) return f(std::integral_constant<int, kNoModes>{});
+  if (a.split) return f(std::integral_constant<int, kSplitModes>{});
+  return f(std::integral_constant<int, kModes>{});
+}
+
 // Per-block partial sums of |exact phi - phi| into partial[3 * blocks].
 static int launch_diff(const FieldArgs &a, int precision, const void *phi, double *partial, cudaStream_t st,
                        int *blocks) {
@@ -334,11 +368,12 @@ static int launch_diff(const FieldArgs &a, int precision, const void *phi, doubl
     if (rc == FF_OK) fn<<<*blocks, kSumThreads, smem, st>>>(a, t, p, partial);
     return rc;
   };
-  const bool m = a.nmodes > 0;
   const double *pd = static_cast<const double *>(phi);
   const float *pf = static_cast<const float *>(phi);
-  const int rc = precision == FF_FP64 ? (m ? launch(k_diff<double, true>, pd) : launch(k_diff<double, false>, pd))
-                                      : (m ? launch(k_diff<float, true>, pf) : launch(k_diff<float, false>, pf));
+  const int rc = with_modes(a, [&](auto modes) {
+    constexpr int M = decltype(modes)::value;
+    return precision == FF_FP64 ? launch(k_diff<double, M>, pd) : launch(k_diff<float, M>, pf);
+  });
   if (rc != FF_OK) return rc;
   FF_CUDA(cudaGetLastError());
   return FF_OK;
@@ -461,11 +496,12 @@ int ff_init_field(const int n[3], const double xlo[3], const double dx[3], int n
     if (rc == FF_OK) fn<<<blocks, kSumThreads, smem, st>>>(a, t, p);
     return rc;
   };
-  const bool m = a.nmodes > 0;
   double *pd = static_cast<double *>(f);
   float *pf = static_cast<float *>(f);
-  rc = precision == FF_FP64 ? (m ? launch(k_init<double, true>, pd) : launch(k_init<double, false>, pd))
-                            : (m ? launch(k_init<float, true>, pf) : launch(k_init<float, false>, pf));
+  rc = with_modes(a, [&](auto modes) {
+    constexpr int M = decltype(modes)::value;
+    return precision == FF_FP64 ? launch(k_init<double, M>, pd) : launch(k_init<float, M>, pf);
+  });
   if (rc != FF_OK) return rc;
   FF_CUDA(cudaGetLastError());
   return FF_OK;
