@@ -436,18 +436,14 @@ class SumScratch {
 // reserved the device memory, a time-critical loop where cudaMalloc's implicit
 // device synchronisation is not acceptable, or plug-in code that may not call
 // the CUDA allocator at all.  For them the partial sums live in a fixed
-// file-scope device array instead of a per-call buffer: every GPU that loads
-// this library holds it (about 384 KB) until the process exits.
+// file-scope device array of their own instead of the slots or a per-call buffer:
+// every GPU that loads this library holds it (28 KB) until the process exits.
 //
-// Each block reduces its tiles in a fixed order; the grid is a function of the
-// dimensions alone, so the summation order is the same on every call for a
-// given grid.  The grid is limited to kNoAllocMaxPoints = 2^30 points (1024^3);
-// the array holds the partials of at most kNoAllocMaxChunks blocks plus the
-// final triple.
-constexpr int kNoAllocMaxChunks = 16384;
+// The kernels and the summation order are those of ff_error_sums.  kNoAllocMaxPoints
+// = 2^30 points (1024^3) is the entry point's stated limit; the partials of
+// kSumBlocks blocks would serve any grid.
 constexpr long kNoAllocMaxPoints = 1L << 30;
-static_assert(kSumBlocks <= kNoAllocMaxChunks, "the fixed array holds every block's partials");
-static __device__ __align__(256) double g_noalloc_partials[3 * kNoAllocMaxChunks + 3];
+static __device__ __align__(256) double g_noalloc_partials[kSumSlotDoubles];
 
 // Device address of g_noalloc_partials on the current device.  The name is a
 // host-side stand-in, not a device address, so it is looked up once per
@@ -549,7 +545,7 @@ int ff_error_sums_noalloc(const int n[3], const double xlo[3], const double dx[3
   const long N = (long)n[0] * n[1] * n[2];
   if (N > kNoAllocMaxPoints)
     return set_error(FF_ERR_UNSUPPORTED,
-                     "ff_error_sums_noalloc: %ld points exceed the fixed partial-sum array's limit of %ld points", N,
+                     "ff_error_sums_noalloc: %ld points are above this entry point's limit of %ld points", N,
                      kNoAllocMaxPoints);
   double *partial = nullptr;
   rc = noalloc_partials(&partial);
@@ -559,7 +555,7 @@ int ff_error_sums_noalloc(const int n[3], const double xlo[3], const double dx[3
   int blocks = 0;
   rc = launch_diff(a, precision, phi, partial, st, &blocks);
   if (rc != FF_OK) return rc;
-  double *total = partial + 3 * kNoAllocMaxChunks;
+  double *total = partial + 3 * kSumBlocks;
   k_diff_final<<<1, kSumThreads, 0, st>>>(partial, blocks, total);
   cudaError_t e = cudaGetLastError();
   double host[3] = {0, 0, 0};

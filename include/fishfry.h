@@ -340,7 +340,9 @@ int ff_init_field(const int n[3], const double xlo[3], const double dx[3], int n
  * two-stage reduction.  phi == NULL gives the phi = 0 pass that the reference
  * uses for its relative-norm scales (FishFry.hpp:146-159).  sums is HOST
  * memory; the call waits for the stream, which must belong to the current
- * device (as every stream passed to this library must). */
+ * device (as every stream passed to this library must).  Its partial sums live
+ * in one of 16 slots inside the library (455 KB per GPU, held until the process
+ * exits); a call that finds all of them in use by other threads allocates. */
 int ff_error_sums(const int n[3], const double xlo[3], const double dx[3], int nmodes,
                   const ff_mode *modes, int precision, const void *phi, double sums[3], void *stream);
 
@@ -349,11 +351,11 @@ int ff_error_sums(const int n[3], const double xlo[3], const double dx[3], int n
  * want the norms: their host application's pool allocator already holds the
  * device memory, cudaMalloc's implicit synchronisation is unacceptable in their
  * loop, or they are plug-ins that may not call the CUDA allocator at all.
- * This entry point calls no cudaMalloc/cudaFree: its partial sums live in a
- * fixed device array inside the library (about 384 KB per GPU, held until the
- * process exits), and grids are limited to 2^30 points (1024^3); larger ones
- * return FF_ERR_UNSUPPORTED.  Same arguments and results as ff_error_sums,
- * summed in a different fixed order (so sums agree to rounding, max exactly).
+ * This entry point calls no cudaMalloc/cudaFree, however many calls are under
+ * way: its partial sums live in a fixed device array of its own inside the
+ * library (28 KB per GPU, held until the process exits).  It takes grids of up to
+ * 2^30 points (1024^3); larger ones return FF_ERR_UNSUPPORTED.  Same arguments
+ * and results as ff_error_sums, summed in the same fixed order.
  * The first call on each device looks up that array's device address and
  * remembers it; make that call before any stream capture, and do not use this
  * entry point after a cudaDeviceReset in the same process (the remembered
