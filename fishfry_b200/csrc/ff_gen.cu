@@ -168,9 +168,8 @@ template <typename C> __global__ void k_gen_twiddles(const TableStages t, C *tw)
 
 }  // namespace
 
-size_t gen_axis_bytes(int n, int esz) {
-  // at most 8 stages of n/R * (R+1) values
-  return r256((size_t)kGenMaxStages * (3 * (size_t)n / 2 + 2) * 2 * esz);
+size_t gen_axis_bytes(int n, const std::vector<int> &radix, int esz) {
+  return r256((size_t)gen_table_size(n, radix) * 2 * esz);
 }
 
 void gen_index(int n, const std::vector<int> &radix, int pad, bool by_frequency, std::vector<int> *out) {

@@ -117,7 +117,7 @@ void gen_index(int n, const std::vector<int> &radix, int pad, bool by_frequency,
 
 // Fills the twiddle table of one axis at `mem` (gen_axis_bytes) on the default
 // stream and points ax at it and at the device copy of its index table.
-size_t gen_axis_bytes(int n, int esz);
+size_t gen_axis_bytes(int n, const std::vector<int> &radix, int esz);
 template <typename C> int gen_axis_build(int n, const std::vector<int> &radix, void *mem, const int *idx, GenAxis<C> *ax);
 
 // Raises the pass kernel's shared-memory limit; FF_ERR_UNSUPPORTED if it does

@@ -899,7 +899,7 @@ int ff_plan_create(const int n[3], const double lo[3], const double hi[3], int p
     if (!p->gen[d] && !p->bsM[d]) continue;
     const bool split = p->gen[d] && d == 2;
     gradix[d] = gen_radices(len[d], split);
-    o_gen[d] = take(gen_axis_bytes(len[d], (int)csz / 2));
+    o_gen[d] = take(gen_axis_bytes(len[d], gradix[d], (int)csz / 2));
     gen_index(len[d], gradix[d], split ? gen_pad(len[d], gradix[d]) : 0, split, &gidx[d]);
   }
   // the integer tables, one upload
