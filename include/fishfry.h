@@ -213,7 +213,7 @@ typedef struct ff_server ff_server;
 
 typedef struct {
   size_t hbm_budget; /* bytes reserved for request buffers (2 x ff_plan_bytes per request) */
-  int max_active;    /* requests admitted at once (descriptor slots per precision) */
+  int max_active;    /* requests admitted at once per precision (descriptor slots grow up to it) */
 } ff_server_config;
 
 typedef struct {
