@@ -884,10 +884,14 @@ int ff_plan_create(const int n[3], const double lo[3], const double hi[3], int p
       return set_error(FF_ERR_UNSUPPORTED, "ff_plan_create: too many stages");
     }
     rev[d] = plan_digit_reversal(L, radix[d]);
-    // FP64 compile-time tables start on 16 KB: every SM reads their few lines all the
-    // time, and how those spread over the L2 depends on the address (512-point y
-    // tables 8, 12, 16, 20, 24, 32 KB into the plan: 363, 369, 346, 373, 367, 373 us for
-    // the forward y pass of 512^3, and 354 at 16 KB against 373-389 in 1024x512x256)
+    // FP64 compile-time tables lie at multiples of 16 KB in the plan's block, which
+    // puts the y table 16 KB in.  That is the place that was fast for the first plan
+    // of a process, the one most programs make: 512^3 y passes 346 / 343 us against
+    // 363 / 351 at 8 KB, alike in every fresh process and on two machines (12, 20,
+    // 24 and 32 KB are like 8).  It secures nothing more.  What counts is the table's
+    // physical address: of 128 plans, 32 in a process, six are 3 % faster than the
+    // others (four of 64 with this rule, two of 64 without), and of 16 offsets from
+    // blocks on 2 MB none is fast in three blocks of three.
     if (precision == FF_FP64 && special_n(n[d])) off = (off + 16383) & ~size_t(16383);
     o_tw[d] = take(L * csz);
     o_tw64[d] = precision == FF_FP64 ? o_tw[d] : take(L * sizeof(double2));
