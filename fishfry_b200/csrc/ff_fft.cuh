@@ -49,6 +49,9 @@ template <> __device__ __forceinline__ float2 csub(float2 a, float2 b) {
   return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a);
 }
 template <> __device__ __forceinline__ float2 cscale(float2 a, float s) { return __fmul2_rn(a, make_float2(s, s)); }
+// c + s*a
+__device__ __forceinline__ double2 cfma(double2 a, double s, double2 c) { return mk(fma(a.x, s, c.x), fma(a.y, s, c.y)); }
+__device__ __forceinline__ float2 cfma(float2 a, float s, float2 c) { return __ffma2_rn(a, make_float2(s, s), c); }
 // a*b
 template <typename C> __device__ __forceinline__ C cmul(C a, C b) {
   return mk(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -202,7 +205,11 @@ template <bool INV, typename C> struct Dft<8, INV, C> {
   }
 };
 
-// 16 = 4 x 4: r = 4 r1 + r2, s = s1 + 4 s2, factors w16^(r2 s1) between.
+// 16 = 4 x 4: r = 4 r1 + r2, s = s1 + 4 s2, factors w16^(r2 s1) between; those of
+// 45 degrees, (1 -+ i) sqrt(1/2), keep their sqrt(1/2) for the second transforms'
+// sums, which take it as multiply-adds: one rounding fewer on a quarter of the
+// values, with which a stage of 16 rounds no more than the stages of 8 and 2 that it
+// replaces.
 // cos and sin of pi / 8
 #define FF_C16_1 0.92387953251128675612818318939678828682
 #define FF_S16_1 0.38268343236508977172845998403039886676
@@ -210,6 +217,17 @@ template <bool INV, typename C> struct Dft<16, INV, C> {
   // v * (c -+ i s)
   template <typename T> static __device__ __forceinline__ C rot(C v, T c, T s) {
     return cmul(v, mk(c, INV ? s : -s));
+  }
+  // frequencies q, q + 4, q + 8, q + 12 from a, b, sqrt(1/2) x, d (q = 1, 3)
+  static __device__ __forceinline__ void odd(C *v, int q, C a, C b, C x, C d) {
+    using T = typename Real<C>::type;
+    const T h = (T)FF_SQRT1_2;
+    const C t0 = cfma(x, h, a), t1 = cfma(x, -h, a);
+    const C t2 = cadd(b, d), t3 = mul_wi<INV>(csub(b, d));
+    v[q] = cadd(t0, t2);
+    v[q + 4] = cadd(t1, t3);
+    v[q + 8] = csub(t0, t2);
+    v[q + 12] = csub(t1, t3);
   }
   static __device__ __forceinline__ void run(C *v) {
     using T = typename Real<C>::type;
@@ -221,22 +239,21 @@ template <bool INV, typename C> struct Dft<16, INV, C> {
       for (int r = 0; r < 4; r++) t[q][r] = v[4 * r + q];
       Dft<4, INV, C>::run(t[q]);
     }
-    t[1][1] = rot(t[1][1], c, s);
-    t[1][2] = cscale(cadd(t[1][2], mul_wi<INV>(t[1][2])), h);
-    t[1][3] = rot(t[1][3], s, c);
-    t[2][1] = cscale(cadd(t[2][1], mul_wi<INV>(t[2][1])), h);
-    t[2][2] = mul_wi<INV>(t[2][2]);
-    t[2][3] = cscale(csub(mul_wi<INV>(t[2][3]), t[2][3]), h);
-    t[3][1] = rot(t[3][1], s, c);
-    t[3][2] = cscale(csub(mul_wi<INV>(t[3][2]), t[3][2]), h);
-    t[3][3] = rot(t[3][3], -c, -s);
+    auto plus = [](C z) { return cadd(z, mul_wi<INV>(z)); };    // z (1 -+ i)
+    auto minus = [](C z) { return csub(mul_wi<INV>(z), z); };   // z (-1 -+ i)
+    C y[4] = {t[0][0], t[1][0], t[2][0], t[3][0]};
+    Dft<4, INV, C>::run(y);
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      C y[4] = {t[0][q], t[1][q], t[2][q], t[3][q]};
-      Dft<4, INV, C>::run(y);
-#pragma unroll
-      for (int r = 0; r < 4; r++) v[q + 4 * r] = y[r];
-    }
+    for (int r = 0; r < 4; r++) v[4 * r] = y[r];
+    odd(v, 1, t[0][1], rot(t[1][1], c, s), plus(t[2][1]), rot(t[3][1], s, c));
+    odd(v, 3, t[0][3], rot(t[1][3], s, c), minus(t[2][3]), rot(t[3][3], -c, -s));
+    const C t2 = mul_wi<INV>(t[2][2]), x1 = plus(t[1][2]), x3 = minus(t[3][2]);
+    const C t0 = cadd(t[0][2], t2), t1 = csub(t[0][2], t2);
+    const C p = cadd(x1, x3), m = mul_wi<INV>(csub(x1, x3));
+    v[2] = cfma(p, h, t0);
+    v[6] = cfma(m, h, t1);
+    v[10] = cfma(p, -h, t0);
+    v[14] = cfma(m, -h, t1);
   }
 };
 
