@@ -59,6 +59,21 @@ template <bool CONJ> __device__ __forceinline__ FPair ucmul(FPair a, float2 w) {
   return CONJ ? FPair{cmulc(a.a, w), cmulc(a.b, w)} : FPair{cmul(a.a, w), cmul(a.b, w)};
 }
 
+// m + s u and m - s u.  FP32 as two multiply-adds, which round once each (the
+// negated u costs what the product did: FFMA2 takes no negated operands, and a
+// second constant of either sign took registers that the last stages spilled:
+// 480x400x360 FP32 y 139 / 137 -> 145 / 150 us); FP64 as a product, a sum and a
+// difference (multiply-adds there lengthen the chain: 500^3 z 452 / 459 -> 469 / 475).
+__device__ __forceinline__ void upm(double2 m, double2 u, double s, double2 &p, double2 &q) {
+  const double2 w = uscale(u, s);
+  p = uadd(m, w);
+  q = usub(m, w);
+}
+__device__ __forceinline__ void upm(FPair m, FPair u, float s, FPair &p, FPair &q) {
+  p = ufma(u, s, m);
+  q = ufma(uscale(u, -1.0f), s, m);
+}
+
 template <typename V> struct UReal;
 template <> struct UReal<double2> { using type = double; };
 template <> struct UReal<FPair> { using type = float; };
@@ -86,11 +101,10 @@ template <bool INV, typename V> struct UDft<2, INV, V> {
 template <bool INV, typename V> __device__ __forceinline__ void udft3(V &v0, V &v1, V &v2) {
   using T = typename UReal<V>::type;
   const V t = uadd(v1, v2);
-  const V u = umul_wi<INV>(uscale(usub(v1, v2), (T)FF_SQRT3_2));
+  const V u = umul_wi<INV>(usub(v1, v2));
   const V m = ufma(t, (T)-0.5, v0);
   v0 = uadd(v0, t);
-  v1 = uadd(m, u);
-  v2 = usub(m, u);
+  upm(m, u, (T)FF_SQRT3_2, v1, v2);
 }
 template <bool INV, typename V> __device__ __forceinline__ void udft4(V &v0, V &v1, V &v2, V &v3) {
   const V t0 = uadd(v0, v2), t1 = usub(v0, v2);
@@ -183,18 +197,16 @@ template <bool INV, typename V> struct UDft<8, INV, V> {
     udft4<INV>(v[1], v[3], v[5], v[7]);
     // w8^s = exp(-+i pi s / 4): (o -+ i o)/sqrt 2, -+i, ...
     const T h = (T)FF_SQRT1_2;
-    const V o1 = uscale(uadd(v[3], umul_wi<INV>(v[3])), h);
+    const V o1 = uadd(v[3], umul_wi<INV>(v[3]));   // times sqrt 2
     const V o2 = umul_wi<INV>(v[5]);
-    const V o3 = uscale(usub(umul_wi<INV>(v[7]), v[7]), h);
+    const V o3 = usub(umul_wi<INV>(v[7]), v[7]);   // times sqrt 2
     const V e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1];
     v[0] = uadd(e0, o0);
     v[4] = usub(e0, o0);
-    v[1] = uadd(e1, o1);
-    v[5] = usub(e1, o1);
+    upm(e1, o1, h, v[1], v[5]);
     v[2] = uadd(e2, o2);
     v[6] = usub(e2, o2);
-    v[3] = uadd(e3, o3);
-    v[7] = usub(e3, o3);
+    upm(e3, o3, h, v[3], v[7]);
   }
 };
 // 9 = 3 x 3: r = r1 + 3 r2, s = 3 s1 + s2, factors w9^(r1 s2) between.
