@@ -56,7 +56,7 @@ struct ff_batch {
   unsigned char *desc_host = nullptr;   // pinned image of the descriptors
   CUtensorMap *maps = nullptr;          // device: two tensor maps per grid (y, x boxes of its potential)
   CUtensorMap *maps_host = nullptr;     // pinned image
-  int2 *entries[5] = {};
+  int *entries[5] = {};
   int *starts[5] = {};
   int ntiles[5] = {};
   int ahead[5] = {};             // blocks resident at once
@@ -128,8 +128,8 @@ size_t batch_shape_smem(int precision, const BatchGridHost &g, int kind, const T
 }
 
 // z passes of a runtime length may move line blocks by bulk copies when the
-// lines are 16-byte multiples and the plan has two or more stages (the tile
-// stages its input in the buffer the last stage writes).
+// lines are 16-byte multiples and the plan has two or more stages (lines of one
+// stage, up to 8 points, are left to the threads).
 bool batch_z_bulk_ok(int precision, int nk) {
   return ((size_t)nk * (precision == FF_FP64 ? 8 : 4)) % 16 == 0 && plan_stages(nk) >= 2;
 }
@@ -351,11 +351,11 @@ int build_work(ff_batch *b) {
     if (rc != FF_OK) return rc;
   }
   for (int k = 0; k < 5; k++) {
-    std::vector<int2> ent(b->count);
+    std::vector<int> ent(b->count);
     std::vector<int> start(b->count + 1, 0);
     size_t smem = 256;
     for (int g = 0; g < b->count; g++) {
-      ent[g] = make_int2(g, k);
+      ent[g] = g;
       start[g + 1] = start[g] + batch_tiles_of(b->grids[g], k);
       smem = std::max(smem, batch_shape_smem(b->precision, b->grids[g], k, b->grids[g].shape[k]));
     }
@@ -366,7 +366,7 @@ int build_work(ff_batch *b) {
     if (rc != FF_OK) return rc;
     if (per_sm < 1) return set_error(FF_ERR_UNSUPPORTED, "batch pass %d: a tile does not fit on an SM", k);
     b->ahead[k] = per_sm * b->num_sms;
-    FF_CUDA(cudaMemcpy(b->entries[k], ent.data(), ent.size() * sizeof(int2), cudaMemcpyHostToDevice));
+    FF_CUDA(cudaMemcpy(b->entries[k], ent.data(), ent.size() * sizeof(int), cudaMemcpyHostToDevice));
     FF_CUDA(cudaMemcpy(b->starts[k], start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice));
   }
   b->desc_dirty = true;
@@ -471,15 +471,6 @@ int time_pass(ff_batch *b, int kind, cudaStream_t st, int reps, float *ms) {
   return FF_OK;
 }
 
-}  // namespace
-}  // namespace ff
-
-extern "C" {
-
-}  // extern "C"
-
-namespace ff {
-namespace {
 
 // The batched grids' tables, descriptors, work lists and events (count >= 1
 // grids that batch_check_dims accepted).  On failure the caller destroys b.
@@ -501,7 +492,7 @@ int batch_create_core(ff_batch *b, int count, const int *dims, const double *lo,
   const size_t o_maps = take((size_t)count * 2 * sizeof(CUtensorMap));
   size_t o_ent[5], o_start[5];
   for (int k = 0; k < 5; k++) {
-    o_ent[k] = take((size_t)count * sizeof(int2));
+    o_ent[k] = take((size_t)count * sizeof(int));
     o_start[k] = take((size_t)(count + 1) * sizeof(int));
   }
   b->dmem_size = off;
@@ -520,7 +511,7 @@ int batch_create_core(ff_batch *b, int count, const int *dims, const double *lo,
   b->desc = base + o_desc;
   b->maps = reinterpret_cast<CUtensorMap *>(base + o_maps);
   for (int k = 0; k < 5; k++) {
-    b->entries[k] = reinterpret_cast<int2 *>(base + o_ent[k]);
+    b->entries[k] = reinterpret_cast<int *>(base + o_ent[k]);
     b->starts[k] = reinterpret_cast<int *>(base + o_start[k]);
   }
   int rc = FF_OK;

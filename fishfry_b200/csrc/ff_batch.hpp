@@ -51,10 +51,10 @@ constexpr int kBatchPadRows = 7;
 constexpr int kBatchStages = 6;
 
 // One launch: tiles of entries e = 0..nentry-1 are numbered start[e] ..
-// start[e+1]-1; entry e names (grid, pass).  ahead: tiles (blocks) resident at
+// start[e+1]-1; entry e names the grid.  ahead: tiles (blocks) resident at
 // once; the z passes hint the input of the tile that far on into L2.
 struct BatchWork {
-  const int2 *entry;
+  const int *entry;
   const int *start;
   int nentry;
   int ahead;

@@ -455,7 +455,7 @@ __global__ void __launch_bounds__((KIND == 0 || KIND == 4) ? kBatchZThreads : kZ
   }
   const int t = blockIdx.x;
   int first = 0;
-  const int g = wl.entry[batch_entry(wl.start, wl.nentry, t, &first)].x;
+  const int g = wl.entry[batch_entry(wl.start, wl.nentry, t, &first)];
   {
     // descriptor of the tile's grid into shared memory (read-only below)
     constexpr int kHead = sizeof(GridHead<T>) / 16, kKind = sizeof(KindDesc) / 16;
@@ -472,7 +472,7 @@ __global__ void __launch_bounds__((KIND == 0 || KIND == 4) ? kBatchZThreads : kZ
     const int t2 = t + wl.ahead;
     int first2 = 0;
     if (threadIdx.x >= kBatchZThreads - 32 && t2 < (int)gridDim.x) {
-      const GridDesc<T> *G = grids + wl.entry[batch_entry(wl.start, wl.nentry, t2, &first2)].x;
+      const GridDesc<T> *G = grids + wl.entry[batch_entry(wl.start, wl.nentry, t2, &first2)];
       if (threadIdx.x == kBatchZThreads - 32) {
         const int zW = G->k[KIND].shape.W;
         const long nlines = (long)G->h.a.ni * G->h.a.nj;

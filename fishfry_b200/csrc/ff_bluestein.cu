@@ -97,10 +97,6 @@ template <bool RADER, bool POWER, typename C> __device__ __forceinline__ int bs_
   else return __ldg(a.perm + (POWER || q == 0 ? q : a.ax.n - q));
 }
 
-template <typename C> __device__ __forceinline__ GenLane bs_lane(const BsPass<C> &a) {
-  return {(int)threadIdx.x & ((1 << a.lu) - 1), (int)threadIdx.x >> a.lu, (int)blockDim.x >> a.lu};
-}
-
 // R2C along z (ParisPencil.cpp:152-165).
 template <typename T, bool RADER>
 __global__ void __launch_bounds__(256, 3)
@@ -131,7 +127,7 @@ __global__ void __launch_bounds__(256, 3)
     for (int q = nl * a.lp + threadIdx.x; q < lines * a.lp; q += blockDim.x) raw[q] = (T)0;
     __syncthreads();
   }
-  const GenLane ln = bs_lane(a);
+  const GenLane ln = gen_lane(a);
   const T *ra = raw + 2 * ln.c * a.lp;
   const int second = 2 * units * a.lp;
   // point `pos` of two real lines as one complex line
@@ -220,7 +216,7 @@ __global__ void __launch_bounds__(256, 3)
   if (!z_wait(&mbar, a.status, a.wait_iters)) return;
   z_rows_real_ends(a, rows, nl, lines);
   __syncthreads();
-  const GenLane ln = bs_lane(a);
+  const GenLane ln = gen_lane(a);
   const C *ra = rows + 2 * ln.c * a.sp;
   const int second = 2 * units * a.sp;
   // the Hermitian extension (Bluestein: times conj chirp, zero from nk on)
@@ -290,7 +286,7 @@ __global__ void __launch_bounds__(256, 3)
   const int ktiles = (a.nh + W - 1) / W;
   const int o = blockIdx.x / ktiles;
   const int kt = blockIdx.x - o * ktiles;
-  const GenLane ln = bs_lane(a);
+  const GenLane ln = gen_lane(a);
   const int col = kt * W + ln.c * CU;
   // FP32 rows are padded to an even count: a unit whose second column is past
   // nh reads the padding and does not store it

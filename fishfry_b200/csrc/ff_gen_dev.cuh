@@ -163,10 +163,9 @@ __global__ void __launch_bounds__(256, 3)
 // ------------------------------------------------------------- z passes
 // A block holds `units` columns of line pairs: FP64 unit c is the pair of lines
 // (2c, 2c+1); FP32 unit c holds that pair and the pair of lines (2u + 2c,
-// 2u + 2c + 1), u the tile's units, so that lanes on neighbouring units read
-// lines two pitches apart in both precisions.  Two buffers: the tile and the
-// staging area (real lines of pitch lp on one side, spectrum rows of pitch sp
-// on the other).  Lines at or past the end are zero in and not stored.
+// 2u + 2c + 1), u the tile's units.  Two buffers: the tile and the staging area
+// (real lines of pitch lp on one side, spectrum rows of pitch sp on the other).
+// Lines at or past the end are zero in and not stored.
 //
 // FP32: z tiles with butterflies fastest (ff_gen_lines.cuh), whose unpadded
 // staging moves by one copy each way: 480x400x360 z 162 / 160 -> 141 / 143 us,
@@ -218,10 +217,10 @@ __global__ void __launch_bounds__(256, 3)
                const __grid_constant__ GenPass<typename Cplx<T>::type> a) {
   using C = typename Cplx<T>::type;
   using V = typename Unit<C>::type;
-  constexpr int CU = 16 / sizeof(C);      // line pairs per unit
+  static_assert(sizeof(C) == 16, "FP32 takes k_gen_lines");
   extern __shared__ unsigned char smraw[];
   __shared__ __align__(8) uint64_t mbar;
-  const int nk = a.nk, units = 1 << a.lu, lines = 2 * CU * units;
+  const int nk = a.nk, units = 1 << a.lu, lines = 2 * units;
   V *tile = reinterpret_cast<V *>(align128(smraw));
   unsigned char *stage = reinterpret_cast<unsigned char *>(tile + ((((a.tile_rows << a.lu) + 7) >> 3) << 3));
   T *raw = reinterpret_cast<T *>(stage);
@@ -249,15 +248,13 @@ __global__ void __launch_bounds__(256, 3)
   }
   const GenLane ln = gen_lane(a);
   const T *ra = raw + 2 * ln.c * a.lp;
-  const int second = 2 * units * a.lp;   // FP32: the unit's second pair
   auto ld0 = [&](int, int pos, const GenStage &st, V *v, auto tag) {
     constexpr int R = decltype(tag)::value;
     const T *p = ra + pos;
 #pragma unroll
     for (int r = 0; r < R; r++) {
       const T *q = p + r * st.m;
-      if constexpr (CU == 1) v[r] = mk(q[0], q[a.lp]);
-      else v[r] = {mk(q[0], q[a.lp]), mk(q[second], q[second + a.lp])};
+      v[r] = mk(q[0], q[a.lp]);
     }
   };
   const int S = a.ax.S;
@@ -275,7 +272,6 @@ __global__ void __launch_bounds__(256, 3)
   // (2i) go to the staged rows of the pair's lines.
   const GenStage &s = a.ax.st[S - 1];
   C *out = reinterpret_cast<C *>(stage) + 2 * ln.c * a.sp;
-  const int second_out = 2 * units * a.sp;
   const int nR = s.nb;
   const TileLoad<V> ld{tile, a.lu, ln.c};
   with_split_radix(s.R, [&](auto tag) {
@@ -297,16 +293,8 @@ __global__ void __launch_bounds__(256, 3)
         const int k = low ? k0 + r * nR : nk - k0 - r * nR;
         const V p = low ? z1[r] : z2[R - 1 - r], q = low ? z2[R - 1 - r] : z1[r];   // Z[k], Z[n - k]
         const T h = (T)0.5;
-        auto emit = [&](C *o, C zp, C zq) {
-          o[k] = mk(h * (zp.x + zq.x), h * (zp.y - zq.y));
-          o[k + a.sp] = mk(h * (zp.y + zq.y), h * (zq.x - zp.x));
-        };
-        if constexpr (CU == 1) {
-          emit(out, p, q);
-        } else {
-          emit(out, p.a, q.a);
-          emit(out + second_out, p.b, q.b);
-        }
+        out[k] = mk(h * (p.x + q.x), h * (p.y - q.y));
+        out[k + a.sp] = mk(h * (p.y + q.y), h * (q.x - p.x));
       }
     }
   });
@@ -322,10 +310,10 @@ __global__ void __launch_bounds__(256, 3)
                const __grid_constant__ GenPass<typename Cplx<T>::type> a) {
   using C = typename Cplx<T>::type;
   using V = typename Unit<C>::type;
-  constexpr int CU = 16 / sizeof(C);
+  static_assert(sizeof(C) == 16, "FP32 takes k_gen_lines");
   extern __shared__ unsigned char smraw[];
   __shared__ __align__(8) uint64_t mbar;
-  const int nk = a.nk, units = 1 << a.lu, lines = 2 * CU * units;
+  const int nk = a.nk, units = 1 << a.lu, lines = 2 * units;
   V *tile = reinterpret_cast<V *>(align128(smraw));
   unsigned char *stage = reinterpret_cast<unsigned char *>(tile + ((((a.tile_rows << a.lu) + 7) >> 3) << 3));
   C *rows = reinterpret_cast<C *>(stage);
@@ -350,11 +338,10 @@ __global__ void __launch_bounds__(256, 3)
   __syncthreads();
   const GenLane ln = gen_lane(a);
   const C *ra = rows + 2 * ln.c * a.sp;
-  const int second = 2 * units * a.sp;
   auto ld0 = [&](int, int pos0, const GenStage &st, V *v, auto tag) {
     constexpr int R = decltype(tag)::value;
 #pragma unroll
-    for (int r = 0; r < R; r++) v[r] = z_extend<V>(ra, second, a.sp, nk, pos0 + r * st.m);
+    for (int r = 0; r < R; r++) v[r] = z_extend<V>(ra, 0, a.sp, nk, pos0 + r * st.m);
   };
   const int S = a.ax.S;
   if (S > 1) {
@@ -367,7 +354,6 @@ __global__ void __launch_bounds__(256, 3)
   // lines of the pair
   const GenStage &s = a.ax.st[S - 1];
   T *out = reinterpret_cast<T *>(stage) + 2 * ln.c * a.lp;
-  const int second_out = 2 * units * a.lp;
   const TileLoad<V> ld{tile, a.lu, ln.c};
   with_split_radix(s.R, [&](auto tag) {
     constexpr int R = decltype(tag)::value;
@@ -378,15 +364,8 @@ __global__ void __launch_bounds__(256, 3)
       T *o = out + k0;
 #pragma unroll
       for (int r = 0; r < R; r++) {
-        if constexpr (CU == 1) {
-          o[0] = z[r].x;
-          o[a.lp] = z[r].y;
-        } else {
-          o[0] = z[r].a.x;
-          o[a.lp] = z[r].a.y;
-          o[second_out] = z[r].b.x;
-          o[second_out + a.lp] = z[r].b.y;
-        }
+        o[0] = z[r].x;
+        o[a.lp] = z[r].y;
         o += s.nb;
       }
     }

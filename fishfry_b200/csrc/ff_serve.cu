@@ -129,7 +129,7 @@ struct Lane {
   CUtensorMap *maps_host = nullptr;        // pinned image
   std::vector<int> free_slots;
   std::vector<void *> old_dev, old_host;   // outgrown buffers, which steps in flight may still read
-  // ring buffers: per step r and kind k: entries [slots] int2, starts [slots + 1] int
+  // ring buffers: per step r and kind k: entries [slots] int, starts [slots + 1] int
   void *ring_dev = nullptr;
   unsigned char *ring_host = nullptr;
   size_t ring_bytes = 0;                   // one step's block
@@ -187,7 +187,7 @@ namespace {
 
 size_t step_block_bytes(int slots) {
   auto r = [](size_t b) { return (b + 255) & ~size_t(255); };
-  return 5 * (r(slots * sizeof(int2)) + r((slots + 1) * sizeof(int)));
+  return 5 * (r(slots * sizeof(int)) + r((slots + 1) * sizeof(int)));
 }
 
 // Descriptor slots of a new lane, and their growth by doubling up to max_active
@@ -383,15 +383,15 @@ int admit(ff_server *s, std::unique_lock<std::mutex> &lk) {
 // its launches, in ring block r.
 int launch_step(ff_server *s, Lane &L, int r, const std::vector<Request *> &members, int *launches) {
   // compact layout of this step's work lists in ring block r: per kind the
-  // entries (int2) and the prefix sums (int)
+  // entries (slots) and the prefix sums
   int cnt[5] = {0, 0, 0, 0, 0};
   for (const Request *q : members) cnt[q->next_pass]++;
   size_t e_off[5], s_off[5], off = 0;
   for (int k = 0; k < 5; k++) {
     e_off[k] = off;
-    off += cnt[k] * sizeof(int2);
+    off += cnt[k] * sizeof(int);
     s_off[k] = off;
-    off += ((cnt[k] + 1) * sizeof(int) + 7) & ~size_t(7);
+    off += (cnt[k] + 1) * sizeof(int);
   }
   unsigned char *hb = L.ring_host + (size_t)r * L.ring_bytes;
   char *db = static_cast<char *>(L.ring_dev) + (size_t)r * L.ring_bytes;
@@ -413,7 +413,7 @@ int launch_step(ff_server *s, Lane &L, int r, const std::vector<Request *> &memb
     }
     const int k = q.next_pass;
     int *st = reinterpret_cast<int *>(hb + s_off[k]);
-    reinterpret_cast<int2 *>(hb + e_off[k])[fill[k]] = make_int2(q.slot, k);
+    reinterpret_cast<int *>(hb + e_off[k])[fill[k]] = q.slot;
     st[fill[k] + 1] = st[fill[k]] + batch_tiles_of(q.g, k);
     smem[k] = std::max(smem[k], batch_shape_smem(q.precision, q.g, k, q.g.shape[k]));
     fill[k]++;
@@ -438,7 +438,7 @@ int launch_step(ff_server *s, Lane &L, int r, const std::vector<Request *> &memb
   if (kinds > 1) FF_CUDA(cudaEventRecord(L.fork_ev, L.stream));
   for (int k = 0; k < 5; k++) {
     if (!cnt[k]) continue;
-    const BatchWork wl{reinterpret_cast<const int2 *>(db + e_off[k]), reinterpret_cast<const int *>(db + s_off[k]),
+    const BatchWork wl{reinterpret_cast<const int *>(db + e_off[k]), reinterpret_cast<const int *>(db + s_off[k]),
                        cnt[k], batch_blocks_per_sm(k) * s->num_sms};
     const int tiles = reinterpret_cast<int *>(hb + s_off[k])[cnt[k]];
     cudaStream_t ks = kinds > 1 ? L.kstream[k] : L.stream;

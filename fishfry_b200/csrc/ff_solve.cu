@@ -111,7 +111,6 @@ __global__ void __launch_bounds__(kZThreads, 3)
   extern __shared__ unsigned char smraw[];
   __shared__ __align__(8) uint64_t mbar;
   C *sm = reinterpret_cast<C *>(align128(smraw));
-  const int n = N > 0 ? N : (XPASS ? a.ax[0].n : a.ax[1].n);
   const int ktiles = (a.nh + W - 1) / W;
   const int o = blockIdx.x / ktiles, kt = blockIdx.x - o * ktiles;
   if (threadIdx.x == 0) {
@@ -121,7 +120,7 @@ __global__ void __launch_bounds__(kZThreads, 3)
   pdl_start();
   pdl_wait();
   __syncthreads();
-  if (!tma_tile<C, W, XPASS>(&tmap, sm, &mbar, 0, n, box_rows, o, kt, a.status, a.wait_iters)) return;
+  if (!tma_tile<C, W, XPASS>(&tmap, sm, &mbar, 0, N, box_rows, o, kt, a.status, a.wait_iters)) return;
   if (XPASS) {
     x_tile<T, W, N>(&tmap, a, o, kt, box_rows, sm);
   } else {
@@ -297,27 +296,12 @@ __global__ void __launch_bounds__(kZThreads, 3)
   }
 }
 
-// x pass: forward, filter, inverse; one TMA-loaded tile per block.
-template <typename T, int N>
-static void launch_x(const CUtensorMap &map, typename Cplx<T>::type *dst, const PassArgs<T> &a, int box_rows,
-                     int grid, size_t smem, cudaStream_t st) {
-  constexpr int W = 128 / (2 * (int)sizeof(T));
-  k_strided<T, W, true, false, N><<<grid, kZThreads, smem, st>>>(map, dst, a, box_rows);
-}
-
 }  // namespace ff
 
 // ====================================================================== plan
 using namespace ff;
 
 namespace ff {
-
-bool smooth235(int n) {
-  if (n < 1) return false;
-  for (int p : {2, 3, 5})
-    while (n % p == 0) n /= p;
-  return n == 1;
-}
 
 bool smooth2357(int n) {
   if (n < 1) return false;

@@ -26,8 +26,6 @@ int set_error(int status, const char *fmt, ...);
     }                                                                                       \
   } while (0)
 
-// Prime factors 2, 3, 5 only.
-bool smooth235(int n);
 // Prime factors 2, 3, 5 and 7 only (the radices of the FFT stages).
 bool smooth2357(int n);
 
