@@ -24,14 +24,9 @@ struct FieldArgs {
   int ni, nj, nk;
   double xlo, ylo, zlo, dx, dy, dz;
   int nmodes;
-  int split;   // an amplitude is not finite: weights stay apart from the cosines (kSplitModes)
+  int finite;   // every amplitude is
   ff_mode modes[kMaxModes];
 };
-
-// What a kernel is built for: no modes, modes whose weights its tables hold, or
-// modes with a weight that is not finite (cos A cos B - sin A sin B would be inf -
-// inf), which multiplies the point's cosine as the formula has it.
-enum : int { kNoModes = 0, kModes = 1, kSplitModes = 2 };
 
 // Weight of a mode in f or in phi; the zero mode counts as absent.
 __device__ __forceinline__ int mode_k2(const ff_mode &m) { return m.kx * m.kx + m.ky * m.ky + m.kz * m.kz; }
@@ -85,7 +80,7 @@ struct FieldTiles {
 
 // Values of the tile's 16 points of this thread: f (solution = false) or phi,
 // summed as the point-by-point formulas are (FishFry.hpp:44, :87).
-template <int MODES>
+template <bool MODES>
 __device__ __forceinline__ void tile_values(const FieldArgs &a, const double2 *sm, int warp, int lane, bool solution,
                                             double v[kTileWarpLines][2]) {
   const double2 *zf = sm, *lx = sm + kTileK, *ly = lx + kTileLines;
@@ -98,20 +93,10 @@ __device__ __forceinline__ void tile_values(const FieldArgs &a, const double2 *s
     for (int q = 0; q < 2; q++)
       v[l][q] = solution ? x.x * y.x * z[q].x : x.x * y.x * z[q].y + x.x * y.y * z[q].x + x.y * y.x * z[q].x;
   }
-  if constexpr (MODES == kNoModes) return;
+  if constexpr (!MODES) return;
   double s[kTileWarpLines][2] = {};
   for (int m = 0; m < a.nmodes; m++) {
     const double2 b0 = zm[m * kTileK + lane], b1 = zm[m * kTileK + lane + 32];
-    if constexpr (MODES == kSplitModes) {
-      if (mode_k2(a.modes[m]) == 0) continue;
-      const double w = mode_weight(a.modes[m], solution);
-      for (int l = 0; l < kTileWarpLines; l++) {
-        const double2 c = lm[m * kTileLines + warp * kTileWarpLines + l];
-        s[l][0] = fma(w, c.x * b0.x - c.y * b0.y, s[l][0]);
-        s[l][1] = fma(w, c.x * b1.x - c.y * b1.y, s[l][1]);
-      }
-      continue;
-    }
 #pragma unroll
     for (int l = 0; l < kTileWarpLines; l++) {
       const double2 w = lm[m * kTileLines + warp * kTileWarpLines + l];   // weight times (cos A, sin A)
@@ -161,7 +146,7 @@ __device__ __forceinline__ void line_tables(const FieldArgs &a, double2 *sm, lon
       const ff_mode &md = a.modes[q / kTileLines - 2];
       double2 v = make_double2(0.0, 0.0);
       if (mode_k2(md) != 0) {
-        const double w = a.split ? 1.0 : mode_weight(md, solution);
+        const double w = mode_weight(md, solution);
         sincos((double)md.kx * x + (double)md.ky * y + md.theta, &v.y, &v.x);
         v = make_double2(w * v.x, w * v.y);
       }
@@ -170,7 +155,7 @@ __device__ __forceinline__ void line_tables(const FieldArgs &a, double2 *sm, lon
   }
 }
 
-template <typename T, int MODES>
+template <typename T, bool MODES>
 __global__ void __launch_bounds__(kSumThreads, MODES ? 2 : 4) k_init(const FieldArgs a, const FieldTiles t, T *__restrict__ f) {
   extern __shared__ double2 smf[];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -198,19 +183,90 @@ __global__ void __launch_bounds__(kSumThreads, MODES ? 2 : 4) k_init(const Field
   }
 }
 
+// f (solution = false) or phi at point q by the formulas as they stand.
+__device__ __forceinline__ double point_value(const FieldArgs &a, long q, bool solution) {
+  const long line = q / a.nk;
+  const int k = (int)(q - line * a.nk);
+  const int i = (int)(line / a.nj);
+  const int j = (int)(line - (long)i * a.nj);
+  const double x = a.xlo + i * a.dx, y = a.ylo + j * a.dy, z = a.zlo + k * a.dz;
+  const double2 px = factor_x(x), py = factor_y(y), pz = factor_z(z);
+  double v = solution ? px.x * py.x * pz.x   // FishFry.hpp:87, :44
+                      : px.x * py.x * pz.y + px.x * py.y * pz.x + px.y * py.x * pz.x;
+  if (a.nmodes == 0) return v;
+  double s = 0.0;
+  for (int m = 0; m < a.nmodes; m++) {
+    const ff_mode &md = a.modes[m];
+    if (mode_k2(md) == 0) continue;
+    s += mode_weight(md, solution) * cos((double)md.kx * x + (double)md.ky * y + (double)md.kz * z + md.theta);
+  }
+  return v + s;
+}
+
+// Point by point, in place of the tiles' kernels (by_points).
+template <typename T> __global__ void __launch_bounds__(kSumThreads) k_init_points(const FieldArgs a, T *__restrict__ f) {
+  const long N = (long)a.ni * a.nj * a.nk;
+  for (long q = blockIdx.x * (long)kSumThreads + threadIdx.x; q < N; q += (long)gridDim.x * kSumThreads)
+    f[q] = (T)point_value(a, q, false);
+}
+
+// One point's difference (FishFry.hpp:89) into a thread's {sum|d|, sum d^2,
+// max|d|}.  NaN propagates through the max, as the reference's integer atomicMax
+// on the bit pattern does.
+struct DiffSums {
+  double t1 = 0, t2 = 0, tm = 0;
+  __device__ __forceinline__ void add(double exact, double phi) {
+    const double d = fabs(exact - phi);
+    t1 += d;
+    t2 += d * d;
+    tm = (d > tm || d != d) ? d : tm;
+  }
+};
+
+// The block's sums in a fixed tree, into out[0..2].
+__device__ __forceinline__ void block_sums(const DiffSums &t, double *out) {
+  __shared__ double s1[kSumThreads], s2[kSumThreads], sm[kSumThreads];
+  s1[threadIdx.x] = t.t1;
+  s2[threadIdx.x] = t.t2;
+  sm[threadIdx.x] = t.tm;
+  __syncthreads();
+  for (int w = kSumThreads / 2; w > 0; w >>= 1) {
+    if (threadIdx.x < w) {
+      s1[threadIdx.x] += s1[threadIdx.x + w];
+      s2[threadIdx.x] += s2[threadIdx.x + w];
+      const double o = sm[threadIdx.x + w];
+      if (o > sm[threadIdx.x] || o != o) sm[threadIdx.x] = o;
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    out[0] = s1[0];
+    out[1] = s2[0];
+    out[2] = sm[0];
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kSumThreads) k_diff_points(const FieldArgs a, const T *__restrict__ phi,
+                                                             double *__restrict__ partial) {
+  const long N = (long)a.ni * a.nj * a.nk;
+  DiffSums t;
+  for (long q = blockIdx.x * (long)kSumThreads + threadIdx.x; q < N; q += (long)gridDim.x * kSumThreads)
+    t.add(point_value(a, q, true), phi ? (double)phi[q] : 0.0);
+  block_sums(t, partial + 3 * blockIdx.x);
+}
+
 // Stage 1 of the error sums: per-block {sum|d|, sum d^2, max|d|} over the
 // block's tiles, each thread's points in a fixed order, reduced in a fixed
 // tree; the grid is a function of the dimensions alone, so the sums are
-// reproducible.  NaN propagates through the max, as the reference's integer
-// atomicMax on the bit pattern does.
-template <typename T, int MODES>
+// reproducible.
+template <typename T, bool MODES>
 __global__ void __launch_bounds__(kSumThreads, MODES ? 2 : 3) k_diff(const FieldArgs a, const FieldTiles t, const T *__restrict__ phi,
                                                       double *__restrict__ partial) {
-  __shared__ double s1[kSumThreads], s2[kSumThreads], sm[kSumThreads];
   extern __shared__ double2 smf[];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const long nlines = (long)a.ni * a.nj;
-  double t1 = 0, t2 = 0, tm = 0;
+  DiffSums sums;
   for (int chunk = blockIdx.x % t.columns; chunk < t.chunks; chunk += t.columns) {
     const int k0 = chunk * t.kc, kc = min(t.kc, a.nk - k0);
     __syncthreads();
@@ -236,65 +292,25 @@ __global__ void __launch_bounds__(kSumThreads, MODES ? 2 : 3) k_diff(const Field
         const long line = line0 + warp * kTileWarpLines + l;
 #pragma unroll
         for (int q = 0; q < 2; q++) {
-          if (line < nlines && lane + 32 * q < kc) {
-            const double d = fabs(v[l][q] - (double)p[l][q]);   // FishFry.hpp:89
-            t1 += d;
-            t2 += d * d;
-            tm = (d > tm || d != d) ? d : tm;
-          }
+          if (line < nlines && lane + 32 * q < kc) sums.add(v[l][q], (double)p[l][q]);
         }
       }
     }
   }
-  s1[threadIdx.x] = t1;
-  s2[threadIdx.x] = t2;
-  sm[threadIdx.x] = tm;
-  __syncthreads();
-  for (int w = kSumThreads / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      s1[threadIdx.x] += s1[threadIdx.x + w];
-      s2[threadIdx.x] += s2[threadIdx.x + w];
-      const double o = sm[threadIdx.x + w];
-      if (o > sm[threadIdx.x] || o != o) sm[threadIdx.x] = o;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    partial[3 * blockIdx.x + 0] = s1[0];
-    partial[3 * blockIdx.x + 1] = s2[0];
-    partial[3 * blockIdx.x + 2] = sm[0];
-  }
+  block_sums(sums, partial + 3 * blockIdx.x);
 }
 
 // Stage 2: one block folds the per-block partials in a fixed order.
 __global__ void __launch_bounds__(kSumThreads) k_diff_final(const double *__restrict__ partial, int nb,
                                                             double *__restrict__ out) {
-  __shared__ double s1[kSumThreads], s2[kSumThreads], sm[kSumThreads];
-  double t1 = 0, t2 = 0, tm = 0;
+  DiffSums t;
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-    t1 += partial[3 * b];
-    t2 += partial[3 * b + 1];
+    t.t1 += partial[3 * b];
+    t.t2 += partial[3 * b + 1];
     const double o = partial[3 * b + 2];
-    tm = (o > tm || o != o) ? o : tm;
+    t.tm = (o > t.tm || o != o) ? o : t.tm;
   }
-  s1[threadIdx.x] = t1;
-  s2[threadIdx.x] = t2;
-  sm[threadIdx.x] = tm;
-  __syncthreads();
-  for (int w = kSumThreads / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      s1[threadIdx.x] += s1[threadIdx.x + w];
-      s2[threadIdx.x] += s2[threadIdx.x + w];
-      const double o = sm[threadIdx.x + w];
-      if (o > sm[threadIdx.x] || o != o) sm[threadIdx.x] = o;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    out[0] = s1[0];
-    out[1] = s2[0];
-    out[2] = sm[0];
-  }
+  block_sums(t, out);
 }
 
 static int field_args(const int n[3], const double xlo[3], const double dx[3], int nmodes, const ff_mode *modes,
@@ -315,9 +331,10 @@ static int field_args(const int n[3], const double xlo[3], const double dx[3], i
   a.dy = dx[1];
   a.dz = dx[2];
   a.nmodes = nmodes;
+  a.finite = 1;
   for (int m = 0; m < nmodes; m++) {
     a.modes[m] = modes[m];
-    if (!std::isfinite(modes[m].a)) a.split = 1;
+    if (!std::isfinite(modes[m].a)) a.finite = 0;
   }
   return FF_OK;
 }
@@ -338,6 +355,29 @@ static FieldTiles tile_shape(const FieldArgs &a) {
   return t;
 }
 
+// Whether a kernel goes point by point: for amplitudes that are not finite (a
+// weight times cos A cos B - sin A sin B would be inf - inf), and where tiles hold so
+// few points that their tables cost more than the points' own factors and
+// cosines.  Points of a tile below which that is so, with 64 lines and a few points
+// along z (12 million points FP64, tiles / points): the right-hand side without
+// modes 3 points 235 / 223 us, 4 178 / 223; 16 modes 5 points 796 / 725, 6 667 / 725;
+// 64 modes 7 points 2339 / 2214, 8 2054 / 2213; the sums without modes 4 points
+// 284 / 252, 5 235 / 252, with 64 modes 6 3462 / 3152, 7 2983 / 3153.  A few long
+// lines, whose chunks form the z tables anew, need a quarter more points: 64 modes 9
+// lines 2293 / 2213, 10 2067 / 2213.  One line or one point along z takes up to nine
+// times as long in tiles.
+static bool by_points(const FieldArgs &a, const FieldTiles &t, bool sums) {
+  const long nlines = (long)a.ni * a.nj;
+  const long points = nlines < kTileLines ? t.kc * nlines * 4 / 5 : t.kc * kTileLines;
+  const long least = a.nmodes == 0 ? (sums ? 260 : 200) : sums ? 340 + a.nmodes : 330 + a.nmodes * 14 / 5;
+  return !a.finite || points < least;
+}
+// Their grid: up to `most` blocks.
+static unsigned point_blocks(const FieldArgs &a, int most) {
+  const long want = ((long)a.ni * a.nj * a.nk + kSumThreads - 1) / kSumThreads;
+  return (unsigned)(want < most ? want : most);
+}
+
 static size_t tile_smem(const FieldArgs &a) {
   return sizeof(double2) * ((size_t)(1 + a.nmodes) * kTileK + (size_t)(2 + a.nmodes) * kTileLines);
 }
@@ -350,30 +390,25 @@ template <typename F> static int allow_tables(F fn, size_t smem) {
   return FF_OK;
 }
 
-// Calls f with the kernels' form as a constant.
-template <typename F> static int with_modes(const FieldArgs &a, F &&f) {
-  if (a.nmodes == 0) return f(std::integral_constant<int, kNoModes>{});
-  if (a.split) return f(std::integral_constant<int, kSplitModes>{});
-  return f(std::integral_constant<int, kModes>{});
-}
-
 // Per-block partial sums of |exact phi - phi| into partial[3 * blocks].
 static int launch_diff(const FieldArgs &a, int precision, const void *phi, double *partial, cudaStream_t st,
                        int *blocks) {
   const FieldTiles t = tile_shape(a);
   const size_t smem = tile_smem(a);
-  *blocks = t.columns * t.walkers;
+  const bool points = by_points(a, t, true);
+  *blocks = points ? (int)point_blocks(a, kSumBlocks) : t.columns * t.walkers;
   auto launch = [&](auto fn, auto *p) -> int {
     const int rc = allow_tables(fn, smem);
     if (rc == FF_OK) fn<<<*blocks, kSumThreads, smem, st>>>(a, t, p, partial);
     return rc;
   };
-  const double *pd = static_cast<const double *>(phi);
-  const float *pf = static_cast<const float *>(phi);
-  const int rc = with_modes(a, [&](auto modes) {
-    constexpr int M = decltype(modes)::value;
-    return precision == FF_FP64 ? launch(k_diff<double, M>, pd) : launch(k_diff<float, M>, pf);
-  });
+  auto run = [&](auto *p) -> int {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(p)>>;
+    if (!points) return a.nmodes > 0 ? launch(k_diff<T, true>, p) : launch(k_diff<T, false>, p);
+    k_diff_points<T><<<*blocks, kSumThreads, 0, st>>>(a, p, partial);
+    return FF_OK;
+  };
+  const int rc = precision == FF_FP64 ? run(static_cast<const double *>(phi)) : run(static_cast<const float *>(phi));
   if (rc != FF_OK) return rc;
   FF_CUDA(cudaGetLastError());
   return FF_OK;
@@ -486,18 +521,18 @@ int ff_init_field(const int n[3], const double xlo[3], const double dx[3], int n
     return set_error(FF_ERR_INVALID, "ff_init_field: bad precision %d", precision);
   const FieldTiles t = tile_shape(a);
   const size_t smem = tile_smem(a);
-  const unsigned blocks = (unsigned)(t.columns * t.walkers);
   auto launch = [&](auto fn, auto *p) -> int {
     const int rc = allow_tables(fn, smem);
-    if (rc == FF_OK) fn<<<blocks, kSumThreads, smem, st>>>(a, t, p);
+    if (rc == FF_OK) fn<<<t.columns * t.walkers, kSumThreads, smem, st>>>(a, t, p);
     return rc;
   };
-  double *pd = static_cast<double *>(f);
-  float *pf = static_cast<float *>(f);
-  rc = with_modes(a, [&](auto modes) {
-    constexpr int M = decltype(modes)::value;
-    return precision == FF_FP64 ? launch(k_init<double, M>, pd) : launch(k_init<float, M>, pf);
-  });
+  auto run = [&](auto *p) -> int {
+    using T = std::remove_pointer_t<decltype(p)>;
+    if (!by_points(a, t, false)) return a.nmodes > 0 ? launch(k_init<T, true>, p) : launch(k_init<T, false>, p);
+    k_init_points<T><<<point_blocks(a, 8 * kSumBlocks), kSumThreads, 0, st>>>(a, p);
+    return FF_OK;
+  };
+  rc = precision == FF_FP64 ? run(static_cast<double *>(f)) : run(static_cast<float *>(f));
   if (rc != FF_OK) return rc;
   FF_CUDA(cudaGetLastError());
   return FF_OK;
