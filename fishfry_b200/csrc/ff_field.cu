@@ -54,12 +54,13 @@ __device__ __forceinline__ double2 factor_z(double z) {
 // mode's cosine is cos(A + B) = cos A cos B - sin A sin B with A = kx x + ky y
 // + theta of the line and B = kz z of the point, so a tile evaluates sines,
 // cosines and exponentials once per line and once per k, in shared memory,
-// and a point costs its products and two multiply-adds per mode: the kernels
-// are bound by HBM (no modes) or by the FP64 pipe (64 modes), not by nine
-// FP64 transcendentals per point (and one more per mode).  On one
-// B200, 256^3 FP64 without modes, f and both norms (one write, one read of the
-// field and three calls): 1.67-1.97 ms before, 0.145 ms now, of which about
-// 0.06 ms is launch and wait latency.
+// and a point costs its products and two multiply-adds per mode, not nine FP64
+// transcendentals (and one more per mode).  Tables and FP64 arithmetic bound the
+// kernels, not HBM: 256^3 FP64 without modes k_init takes 27 us for 21 us of
+// writes, k_diff 35 us with phi and 33 without reading it.  f and both norms (three
+// calls) point by point 1.67-1.97 ms, so 0.145 ms, of which about 0.06 ms is launch
+// and wait latency.  Grids whose tiles would be mostly empty go point by point
+// (by_points).
 //
 // A block keeps its z chunk (blockIdx.x % columns) and walks the line tiles, so
 // the z tables are formed once per block (once per chunk on lines of more than

@@ -3,11 +3,10 @@
 //
 // The stages are those of ff_gen_stages.cuh.
 //
-// What bounded these passes before was integer work of the plan read at run
-// time: 338 (z) and 180 (y) warp instructions per 32 complex points at
-// 480x400x360 FP64, a fifth of them FP64 (a digit reversal with a remainder by
-// the runtime radix for each output, a quotient for each butterfly, five-factor
-// plans).  So here
+// A plan read at run time costs integer work: a digit reversal with a remainder
+// for each output, a quotient for each butterfly and five-factor plans took
+// 338 (z) and 180 (y) warp instructions per 32 complex points at 480x400x360 FP64, a
+// fifth of them FP64.  So here
 //   - radices go up to 10 (6 and 10 without inner twiddles, by the prime factor
 //     algorithm), which makes three stages of nearly every length up to 1000;
 //   - the butterfly's block and offset advance by additions;
@@ -17,12 +16,12 @@
 //   - twiddles lie per stage as [j][r], one address for a butterfly's factors;
 //   - the z passes fuse the last stage with the real split as the compile-time
 //     ones do, in one form for every radix.
-// One B200, passes z / y / x / y / z: 480x400x360 FP64 483 / 328 / 424 / 326 /
-// 581 us before, 243 / 215 / 324 / 211 / 240 now (2.14 -> 1.23 ms a solve, 70 %
-// of the copy rate over the five passes' bytes); FP32 332 / 229 / 301 / 232 / 369
-// -> 162 / 137 / 206 / 138 / 160 us (1.46 -> 0.80 ms).
+// One B200, passes z / y / x / y / z with and without all that: 480x400x360 FP64
+// 483 / 328 / 424 / 326 / 581 us -> 250 / 222 / 345 / 214 / 241 (2.14 -> 1.27 ms a
+// solve, 67 % of the copy rate over the five passes' bytes); FP32 332 / 229 / 301 /
+// 232 / 369 -> 137 / 137 / 205 / 136 / 144 (1.46 -> 0.76 ms).
 //
-// What bounds them now: no pipe is saturated (480x400x360 FP64 y pass: DRAM 60 %,
+// What bounds them: no pipe is saturated (480x400x360 FP64 y pass: DRAM 60 %,
 // L1 55 %, FP64 32 %, issue 37 %); a block's load, its stages and its stores
 // follow one another, and 24 warps on an SM (80 registers) overlap them across
 // blocks.  Persistent blocks with two tile buffers, so that no warp waits for a
