@@ -131,11 +131,7 @@ __global__ void __launch_bounds__(256, 3)
   const T *ra = raw + 2 * ln.c * a.lp;
   const int second = 2 * units * a.lp;
   // point `pos` of two real lines as one complex line
-  auto pair = [&](int pos) -> V {
-    const T *q = ra + pos;
-    if constexpr (CU == 1) return mk(q[0], q[a.lp]);
-    else return {mk(q[0], q[a.lp]), mk(q[second], q[second + a.lp])};
-  };
+  auto pair = [&](int pos) { return unit_of<V>(ra + pos, a.lp, second); };
   // Rader: in the root's order; Bluestein: times the chirp, zero from nk on
   auto ld0 = [&](int, int pos0, const GenStage &st, V *v, auto tag) {
     constexpr int R = decltype(tag)::value;
@@ -171,17 +167,7 @@ __global__ void __launch_bounds__(256, 3)
       p = ucmul<false>(tile[(k << a.lu) + ln.c], __ldg(a.chirp + k));
       q = ucmul<false>(tile[(kr << a.lu) + ln.c], __ldg(a.chirp + kr));
     }
-    const T h = (T)0.5;
-    auto emit = [&](C *o, C zp, C zq) {
-      o[k] = mk(h * (zp.x + zq.x), h * (zp.y - zq.y));
-      o[k + a.sp] = mk(h * (zp.y + zq.y), h * (zq.x - zp.x));
-    };
-    if constexpr (CU == 1) {
-      emit(out, p, q);
-    } else {
-      emit(out, p.a, q.a);
-      emit(out + second_out, p.b, q.b);
-    }
+    unit_split(out + k, a.sp, second_out, p, q);
   }
   fence_proxy_async_smem();
   __syncthreads();
@@ -225,26 +211,15 @@ __global__ void __launch_bounds__(256, 3)
 #pragma unroll
     for (int r = 0; r < R; r++) {
       const int pos = pos0 + r * st.m;
-      if constexpr (RADER) v[r] = z_extend<V>(ra, second, a.sp, nk, bs_at<true, false>(a, pos));
-      else if (pos < nk) v[r] = ucmul<true>(z_extend<V>(ra, second, a.sp, nk, pos), __ldg(a.chirp + pos));
+      if constexpr (RADER) v[r] = unit_extend<V>(ra, a.sp, second, nk, bs_at<true, false>(a, pos));
+      else if (pos < nk) v[r] = ucmul<true>(unit_extend<V>(ra, a.sp, second, nk, pos), __ldg(a.chirp + pos));
       else v[r] = zero_unit((V *)nullptr);
     }
   };
   // points k < n (Bluestein: times conj chirp) to the real lines of the pairs
   T *out = reinterpret_cast<T *>(stage) + 2 * ln.c * a.lp;
   const int second_out = 2 * units * a.lp;
-  auto store = [&](int k, V z) {
-    T *o = out + k;
-    if constexpr (CU == 1) {
-      o[0] = z.x;
-      o[a.lp] = z.y;
-    } else {
-      o[0] = z.a.x;
-      o[a.lp] = z.a.y;
-      o[second_out] = z.b.x;
-      o[second_out + a.lp] = z.b.y;
-    }
-  };
+  auto store = [&](int k, V z) { unit_put(out + k, a.lp, second_out, z); };
   auto put = [&](int, int pos0, const GenStage &st, const V *v, auto tag) {
     constexpr int R = decltype(tag)::value;
 #pragma unroll
@@ -255,7 +230,7 @@ __global__ void __launch_bounds__(256, 3)
     }
   };
   V *first = tile + (a.ax.n << a.lu) + ln.c;
-  if (RADER && ln.b0 == 0) *first = z_extend<V>(ra, second, a.sp, nk, 0);
+  if (RADER && ln.b0 == 0) *first = unit_extend<V>(ra, a.sp, second, nk, 0);
   bs_conv<BsWay, RADER, true>(a, ln, tile, ld0, put);
   if (RADER && ln.b0 == 0) store(0, *first);
   fence_proxy_async_smem();

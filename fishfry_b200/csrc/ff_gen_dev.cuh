@@ -17,8 +17,8 @@
 //   - the z passes fuse the last stage with the real split as the compile-time
 //     ones do, in one form for every radix.
 // One B200, passes z / y / x / y / z with and without all that: 480x400x360 FP64
-// 483 / 328 / 424 / 326 / 581 us -> 250 / 222 / 345 / 214 / 241 (2.14 -> 1.27 ms a
-// solve, 67 % of the copy rate over the five passes' bytes); FP32 332 / 229 / 301 /
+// 483 / 328 / 424 / 326 / 581 us -> 236 / 222 / 345 / 214 / 241 (2.14 -> 1.26 ms a
+// solve, 68 % of the copy rate over the five passes' bytes); FP32 332 / 229 / 301 /
 // 232 / 369 -> 137 / 137 / 205 / 136 / 144 (1.46 -> 0.76 ms).
 //
 // What bounds them: no pipe is saturated (480x400x360 FP64 y pass: DRAM 60 %,
@@ -251,10 +251,7 @@ __global__ void __launch_bounds__(256, 3)
     constexpr int R = decltype(tag)::value;
     const T *p = ra + pos;
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-      const T *q = p + r * st.m;
-      v[r] = mk(q[0], q[a.lp]);
-    }
+    for (int r = 0; r < R; r++) v[r] = unit_of<V>(p + r * st.m, a.lp, 0);
   };
   const int S = a.ax.S;
   if (S > 1) {
@@ -291,9 +288,7 @@ __global__ void __launch_bounds__(256, 3)
         const bool low = 2 * r < R;
         const int k = low ? k0 + r * nR : nk - k0 - r * nR;
         const V p = low ? z1[r] : z2[R - 1 - r], q = low ? z2[R - 1 - r] : z1[r];   // Z[k], Z[n - k]
-        const T h = (T)0.5;
-        out[k] = mk(h * (p.x + q.x), h * (p.y - q.y));
-        out[k + a.sp] = mk(h * (p.y + q.y), h * (q.x - p.x));
+        unit_split(out + k, a.sp, 0, p, q);
       }
     }
   });
@@ -340,7 +335,7 @@ __global__ void __launch_bounds__(256, 3)
   auto ld0 = [&](int, int pos0, const GenStage &st, V *v, auto tag) {
     constexpr int R = decltype(tag)::value;
 #pragma unroll
-    for (int r = 0; r < R; r++) v[r] = z_extend<V>(ra, 0, a.sp, nk, pos0 + r * st.m);
+    for (int r = 0; r < R; r++) v[r] = unit_extend<V>(ra, a.sp, 0, nk, pos0 + r * st.m);
   };
   const int S = a.ax.S;
   if (S > 1) {
@@ -363,8 +358,7 @@ __global__ void __launch_bounds__(256, 3)
       T *o = out + k0;
 #pragma unroll
       for (int r = 0; r < R; r++) {
-        o[0] = z[r].x;
-        o[a.lp] = z[r].y;
+        unit_put(o, a.lp, 0, z[r]);
         o += s.nb;
       }
     }

@@ -85,6 +85,10 @@ __device__ __forceinline__ void line_dif(const GenStage *st, int s1, const TW &t
   }
 }
 
+// The lines of unit c of a tile.  The same values as unit_of and the like
+// (ff_gen_stages.cuh) form at a lane's fixed unit, addressed from the tile's
+// start: written in terms of those the kernels here lost (480x400x360 FP32 z
+// inverse 144 -> 153 to 163 us, 48 grids of ragged lengths FP64 999 -> 1009).
 // Point pos of unit c of staged real lines as complex values.
 template <typename V, typename T> __device__ __forceinline__ V line_pair(const T *raw, int nk, int units, int c, int pos) {
   const T *q = raw + 2 * c * nk + pos;

@@ -554,18 +554,54 @@ __device__ __forceinline__ void z_rows_real_ends(const GenPass<C> &a, C *rows, i
   }
 }
 
-// Point pos of the Hermitian extension of a unit's line pairs (row a of a pair
-// at q, row b a pitch behind; FP32: the second pair `second` further): Z[k] =
-// A[k] + i B[k] up to n/2, conj A[n-k] + i conj B[n-k] above.
+// Lines of a unit in staged memory: a pair's second line lies `pitch` behind its
+// first; FP32's second pair `second` behind the first pair.
+// Two real lines at q as one complex line, and back.
+template <typename V, typename T> __device__ __forceinline__ V unit_of(const T *q, int pitch, int second) {
+  if constexpr (sizeof(T) == 8) return mk(q[0], q[pitch]);
+  else return {mk(q[0], q[pitch]), mk(q[second], q[second + pitch])};
+}
+template <typename V, typename T> __device__ __forceinline__ void unit_put(T *q, int pitch, int second, V v) {
+  if constexpr (sizeof(T) == 8) {
+    q[0] = v.x;
+    q[pitch] = v.y;
+  } else {
+    q[0] = v.a.x;
+    q[pitch] = v.a.y;
+    q[second] = v.b.x;
+    q[second + pitch] = v.b.y;
+  }
+}
+
+// A[k] = (Z[k] + conj Z[n-k]) / 2 and B[k] = (Z[k] - conj Z[n-k]) / (2i), p = Z[k],
+// q = Z[n-k], to the rows at o of the unit's lines (ParisPencil.cpp:152-165).
+template <typename V, typename C> __device__ __forceinline__ void unit_split(C *o, int pitch, int second, V p, V q) {
+  using T = typename Real<C>::type;
+  const T h = (T)0.5;
+  auto emit = [&](C *r, C zp, C zq) {
+    r[0] = mk(h * (zp.x + zq.x), h * (zp.y - zq.y));
+    r[pitch] = mk(h * (zp.y + zq.y), h * (zq.x - zp.x));
+  };
+  if constexpr (sizeof(C) == 16) {
+    emit(o, p, q);
+  } else {
+    emit(o, p.a, q.a);
+    emit(o + second, p.b, q.b);
+  }
+}
+
+// Point pos of the Hermitian extension of a unit's rows (row a of a pair at q, row
+// b a pitch behind): Z[k] = A[k] + i B[k] up to n/2, conj A[n-k] + i conj B[n-k]
+// above (ParisPencil.cpp:368-380).
 template <typename V, typename C>
-__device__ __forceinline__ V z_extend(const C *ra, int second, int sp, int nk, int pos) {
+__device__ __forceinline__ V unit_extend(const C *ra, int pitch, int second, int nk, int pos) {
   using T = typename Real<C>::type;
   const bool lo = 2 * pos <= nk;
   const C *q = ra + (lo ? pos : nk - pos);
   const T s = lo ? (T)1 : (T)-1;
   auto join = [&](C sa, C sb) { return mk(fma(-s, sb.y, sa.x), fma(s, sa.y, sb.x)); };
-  if constexpr (sizeof(C) == 16) return join(q[0], q[sp]);
-  else return {join(q[0], q[sp]), join(q[second], q[second + sp])};
+  if constexpr (sizeof(C) == 16) return join(q[0], q[pitch]);
+  else return {join(q[0], q[pitch]), join(q[second], q[second + pitch])};
 }
 
 }  // namespace ff
