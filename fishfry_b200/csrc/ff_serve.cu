@@ -332,7 +332,8 @@ int start_request(ff_server *s, Request &q) {
 // Admission of pending requests in arrival order; a request that does not
 // fit now is passed over (later, smaller ones may fit) and retried when
 // memory or slots are freed.  At most kAdmitWindow queued requests are
-// examined per pass, so a long queue costs nothing while the budget is full.
+// examined per pass, so a long queue costs nothing while the budget is full; a
+// pass that admitted some is followed by another if the queue goes on behind them.
 constexpr int kAdmitWindow = 64;
 
 // The bookkeeping runs under the caller's lock; the device work (tables, input
@@ -341,7 +342,8 @@ constexpr int kAdmitWindow = 64;
 int admit(ff_server *s, std::unique_lock<std::mutex> &lk) {
   std::vector<Request *> fresh;
   int seen = 0;
-  for (auto it = s->pending.begin(); it != s->pending.end() && seen < kAdmitWindow; seen++) {
+  auto it = s->pending.begin();
+  for (; it != s->pending.end() && seen < kAdmitWindow; seen++) {
     Request &q = s->reqs[*it];
     Lane &L = s->lane[q.precision == FF_FP64 ? 0 : 1];
     size_t od = 0, op = 0;
@@ -369,6 +371,9 @@ int admit(ff_server *s, std::unique_lock<std::mutex> &lk) {
     it = s->pending.erase(it);
   }
   if (fresh.empty()) return FF_OK;
+  // requests behind the window: nothing else may call for the next pass once all
+  // submissions are in and no result is fetched before the last one is done
+  if (it != s->pending.end()) s->admit_dirty = true;
   lk.unlock();
   int rc = FF_OK;
   for (Request *q : fresh) {

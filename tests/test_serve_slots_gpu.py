@@ -39,9 +39,9 @@ def test_requests_beyond_the_first_slots(torch_cuda, ff, count, max_active):
         at = {i: q for q, i in enumerate(ids)}
         if max_active >= count:
             for i in ids:
-                srv.wait(i)
+                srv.wait(i, 60_000.0)
         for _ in range(count):
-            i = srv.next()[0]
+            i = srv.next(60_000.0)[0]
             srv.fetch(i, out[at[i]])
         srv.check()
     finally:
