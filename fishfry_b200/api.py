@@ -234,7 +234,9 @@ class Server:
         return rid.value, info.latency_ms, info.queue_ms, info.run_ms
 
     def fetch(self, rid, out=None, on_host=None):
-        """Copies the potential into `out` (device or host tensor; None: drop) and releases the request."""
+        """Copies the potential into `out` (device or host tensor; None: drop) and releases the request.
+        The copy is not ordered after work pending on other streams: memory that kernels still use (a
+        block that the caching allocator has just handed over, too) has to be synchronised first."""
         if on_host is None:
             on_host = out is not None and not isinstance(out, int) and not out.is_cuda
         check(lib().ff_server_fetch(self._h, int(rid), _ptr(out), int(bool(on_host))), "ff_server_fetch")

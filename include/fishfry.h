@@ -258,7 +258,10 @@ int ff_server_wait(ff_server *server, uint64_t id, double timeout_ms, ff_request
 int ff_server_next(ff_server *server, double timeout_ms, uint64_t *id, ff_request_info *info);
 
 /* Copies a finished request's potential (ni*nj*nk values) to phi (host or
- * device; phi NULL copies nothing) and releases the request's buffers.  While
+ * device; phi NULL copies nothing) and releases the request's buffers.  The copy
+ * runs on the server's own stream and is waited for; work of other streams on a
+ * device phi (an allocator's earlier use of its memory among it) must be complete
+ * before the call.  While
  * the copy runs the request is claimed: a fetch or release of the same id from
  * another thread returns FF_ERR_INVALID, and the buffers are not reused. */
 int ff_server_fetch(ff_server *server, uint64_t id, void *phi, int phi_on_host);
